@@ -768,6 +768,9 @@ void Engine::build_layout() {
         for (int r : order) {
             RepDev& rd = rep_host_[r];
             if (groups_.empty() || std::memcmp(groups_.back().K, rd.K, sizeof(rd.K)) != 0) {
+                // each group starts on 16 bytes (two grids of odd sizes end 8 bytes off):
+                // the kernels read and write grids with rows of 4 n points as float4
+                n_real_ = (n_real_ + 3) & ~3LL;
                 FftGroup g;
                 std::memcpy(g.K, rd.K, sizeof(g.K));
                 g.first_rep = r;

@@ -1,0 +1,33 @@
+"""PME grids of several sizes and factors on the GPU, against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import atmmetaforce as atm
+from atmmetaforce import synthetic as S
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+U_TOL, F_TOL = 0.01, 1e-4  # kJ/mol, force RMS relative: the parity tests' tolerances
+
+
+def _check(grids, diff):
+    cases = []
+    for k, g in enumerate(grids):
+        c = S.water_ligand_box(1100, 2.25, [9], [(1.1, 1.0, 1.2)], S.PME, 0.9, seed=60 + k)
+        c.spec.grid = tuple(g)
+        cases.append(c)
+    b = atm.ReplicaBatch([atm.system_from_case(c)[0] for c in cases], 0, {"DifferencePath": diff})
+    E, F, r = b.evaluate(np.concatenate([c.pos for c in cases]))
+    for k, c in enumerate(cases):
+        ref = O.atm_eval(c.spec, c.pos, c.displ, c.params)
+        f = F[b.offsets[k]:b.offsets[k + 1]]
+        assert abs(r[k]["pert"] - ref["usc"]) <= U_TOL, grids[k]
+        assert np.sqrt(((f - ref["forces"]) ** 2).sum() / (ref["forces"] ** 2).sum()) <= F_TOL, grids[k]
+
+
+@pytest.mark.parametrize("diff", [0, 1], ids=["two-states", "difference"])
+def test_grids_of_odd_and_multiple_of_four_sizes_in_one_batch(diff):
+    """Two grids of an odd size are 2 mod 4 floats long; the next replicas' grids,
+    whose rows are read and written as float4, must start on 16 bytes all the same."""
+    _check([(23, 23, 23), (24, 24, 24), (23, 25, 21), (25, 23, 28), (24, 24, 24)], diff)
