@@ -31,3 +31,11 @@ def test_grids_of_odd_and_multiple_of_four_sizes_in_one_batch(diff):
     """Two grids of an odd size are 2 mod 4 floats long; the next replicas' grids,
     whose rows are read and written as float4, must start on 16 bytes all the same."""
     _check([(23, 23, 23), (24, 24, 24), (23, 25, 21), (25, 23, 28), (24, 24, 24)], diff)
+
+
+@pytest.mark.parametrize("diff", [0, 1], ids=["two-states", "difference"])
+def test_grids_with_prime_factors_beyond_the_dedicated_radices(diff):
+    """The direct DFT stage: primes 11 to 37, one to three past a multiple of its
+    outputs per work item, alone (23, 29, 31, 37) and after other stages (22, 26,
+    33, 34, 38, 39)."""
+    _check([(22, 23, 26), (31, 29, 37), (34, 39, 38), (33, 22, 22), (26, 22, 34)], diff)
