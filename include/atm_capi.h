@@ -189,12 +189,12 @@ int atm_system_set_position_restraints_periodic(atm_system_t sys, int periodic);
  * pair lists and the pair tiles as two kernels; 1: one persistent kernel that
  * builds each row's lists and evaluates its tiles at once; the autotuner chooses
  * between them); SpreadByOwner=0|1 (default 1: PME charges spread once per atom,
- * by the grid brick that holds its stencil base, and the bricks summed into
- * integer grids; 0: every brick spreads each atom whose stencil touches it; the
- * grids, and so every result, are the same bits either way); SpreadBrick=n (the
- * spreading brick edge in grid points, 0: each atom's stencil added straight into
- * the integer grid by atomics; the autotuner chooses among 20, 19, 16, 12 and 0;
- * same bits in every case). */
+ * straight into the integer grids by atomics or, with a brick edge, by the grid
+ * brick that holds its stencil base; 0: every brick spreads each atom whose stencil
+ * touches it; the grids, and so every result, are the same bits either way);
+ * SpreadBrick=n (the spreading brick edge in grid points, 0: no bricks, the default
+ * unless SpreadByOwner=0; the autotuner chooses among 20, 19, 16, 12 and 0; same
+ * bits in every case). */
 int atm_context_create(atm_system_t sys, int device, const char* properties, atm_context_t* out);
 int atm_context_destroy(atm_context_t ctx);
 /* Context::setPositions (host doubles, n x 3, nm). */

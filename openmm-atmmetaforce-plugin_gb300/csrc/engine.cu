@@ -851,16 +851,21 @@ void Engine::build_layout() {
     layout_ready_ = true;
 }
 
-// Spreading bricks: at most tune_brick_ grid points per dimension, two grids per
+// The spreading scheme.  Per atom (k_spread_atoms, int32 grids, so with the
+// hand-written transform only) unless a brick edge or spreading by every touching
+// brick was asked for: its time follows the atoms, where the bricks' follows the
+// longest brick.  us of the kernel, bricks of 16 / per atom: 22 x 23,558 atoms
+// 151 / 93, 8 x 60,000 172 / 94, 8 x 12,000 60 / 23, 1 x 23,558 50 / 11 (in MD,
+// beside the pair tiles).
+// Bricks: at most tune_brick_ (or 16) grid points per dimension, two grids per
 // replica.  Spreading by owner needs the hand-written forward transform (it reads
 // the int32 grids) and grids larger than a brick plus the stencil reach (4 points)
 // in every dimension of every replica, so that a brick's padded accumulator never
-// wraps onto itself.  tune_brick_ 0: spreading per atom (k_spread_atoms, int32
-// grids, also with the hand-written transform only; bricks of 16 otherwise).
+// wraps onto itself.
 void Engine::build_bricks() {
     brick_cta_rep_.clear();
     brick_smem_ = 0;
-    spread_atoms_ = tune_brick_ == 0 && use_fft_;
+    spread_atoms_ = use_fft_ && (tune_brick_ == 0 || (tune_brick_ == kBrickAuto && spread_owner_pref_));
     const int edge = tune_brick_ > 0 ? tune_brick_ : 16;
     spread_owner_ = spread_owner_pref_ && use_fft_;
     for (int r = 0; r < R_; r++) {

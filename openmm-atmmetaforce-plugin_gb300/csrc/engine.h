@@ -191,12 +191,13 @@ private:
     int tile_grid_ = 0;
     int sms_ = 0, max_tile_per_sm_ = 1;
     int tune_tile_per_sm_ = 0;     // 0: as many as fit
-    int tune_brick_ = 16;          // spreading brick edge (grid points)
+    static constexpr int kBrickAuto = -1;
+    int tune_brick_ = kBrickAuto;  // spreading brick edge (grid points), 0: per atom; kBrickAuto: build_bricks' rule
     bool tune_pme_stream_ = true;  // PME on its own stream
     bool tune_fused_ = false;      // lists and pair tiles in one persistent kernel
     bool spread_owner_pref_ = true;  // spreading by owner brick where the grids allow it
     bool spread_owner_ = false;      // ... and in use (build_bricks)
-    bool spread_atoms_ = false;      // spreading per atom (tune_brick_ 0, hand-written transform)
+    bool spread_atoms_ = false;      // spreading per atom in use (build_bricks)
 
     // host copies of the layout
     std::vector<int> orig_, slot_of_, block_rep_, block_cls_;

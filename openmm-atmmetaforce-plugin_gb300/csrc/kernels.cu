@@ -666,19 +666,28 @@ __global__ void __launch_bounds__(kBrickThreads) k_spread(Args a) {
     }
 }
 
-// Spreading per atom, for systems too small to fill the GPU with bricks: a warp
-// takes one block of 32 atoms (grid 0: every block at x; grid 1: every moving
-// block at x with -q and at x + d with +q), each lane computes its atom's stencil,
-// then the atoms one by one with the lanes on the 5 x 5 (y, z) offsets add their
-// 125 points to the int32 grid by atomics.  The integer contribution of an atom to
-// a point is computed exactly as the bricks compute it, so the grids are the same
-// bits.
+// Spreading per atom: a warp takes kSpreadAtoms atoms of a block of 32 (grid 0:
+// every block at x; grid 1: every moving block at x with -q and at x + d with +q), its
+// first lanes compute a stencil each, then the atoms one by one with the lanes on the
+// 5 x 5 (y, z) offsets add their 125 points to the int32 grid by atomics.  The integer
+// contribution of an atom to a point is computed exactly as the bricks compute it,
+// so the grids are the same bits.
+//
+// Bound by the rate at which a warp's atomics leave the SM (about 5 rows of 20
+// bytes each), so by warps until the L2's rate is reached: with a whole block per
+// warp one 23,558-atom box is 744 warps on 93 SMs.  32 / 16 / 8 / 4 atoms per warp,
+// us of the kernel: 1 x 23,558 beside the pair tiles 47 / 21 / 11 / 10, 8 x 12,000
+// 54 / 25 / 23 / 24, 8 x 60,000 97 / 91 / 94 / 108, 22 x 23,558 102 / 93 / 93 / 118
+// (fewer atoms per warp repeat the per-warp set-up).
 constexpr int kSpreadAtomWarps = 8;
+constexpr int kSpreadAtoms = 8;
 
 __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a) {
-    __shared__ float s_st[kSpreadAtomWarps][32 * kStencilWords];
+    __shared__ float s_st[kSpreadAtomWarps][kSpreadAtoms * kStencilWords];
+    constexpr int kParts = kTile / kSpreadAtoms;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int item = blockIdx.x * kSpreadAtomWarps + w;
+    const int part_item = blockIdx.x * kSpreadAtomWarps + w;
+    const int item = part_item / kParts, part = part_item - item * kParts;
     if (item >= a.NB + 2 * a.n_mov_blocks) return;
     int blk, code;  // 0: grid 0 at x; 1: grid 1, -q at x; 3: grid 1, +q at x + d
     if (item < a.NB) {
@@ -690,7 +699,8 @@ __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a) 
         code = (m & 1) ? 3 : 1;
     }
     const RepDev& R = a.reps[a.block_rep[blk]];
-    const int s = blk * kTile + lane;
+    const int at = part * kSpreadAtoms + lane;  // atom of the block (lanes below kSpreadAtoms)
+    const int s = blk * kTile + (min(at, kTile - 1));
     const int nreal = __float_as_int(a.bb_h[blk].w);
     float4 p = a.posq[s];
     if (code == 1) p.w = -p.w;
@@ -701,7 +711,7 @@ __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a) 
         p.z += dd.z;
         wrap3(p.x, p.y, p.z, R);
     }
-    const bool ok = lane < nreal && p.w != 0.0f;
+    const bool ok = lane < kSpreadAtoms && at < nreal && p.w != 0.0f;
     float* st = s_st[w];
     if (ok) {
         Stencil S;
@@ -721,23 +731,22 @@ __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a) 
     const int K0 = R.K[0], K1 = R.K[1], K2 = R.K[2];
     int* G = reinterpret_cast<int*>(a.qreal + R.real_off + (code ? (size_t)K0 * K1 * K2 : 0));
     const int b0 = lane / kOrder, c0 = lane % kOrder;
+    if (lane >= kOrder * kOrder) return;
     while (bal) {
         const int src = __ffs(bal) - 1;
         bal &= bal - 1;
         const float* wv = st + src * kStencilWords;
-        if (lane < kOrder * kOrder) {
-            const int bases = __float_as_int(wv[15]);
-            int y = ((bases >> 10) & 1023) - b0, z = (bases & 1023) - c0;
-            y += y < 0 ? K1 : 0;
-            z += z < 0 ? K2 : 0;
-            const float wyz = wv[kOrder + b0] * wv[2 * kOrder + c0];
-            const int x0 = bases >> 20;
+        const int bases = __float_as_int(wv[15]);
+        int y = ((bases >> 10) & 1023) - b0, z = (bases & 1023) - c0;
+        y += y < 0 ? K1 : 0;
+        z += z < 0 ? K2 : 0;
+        const float wyz = wv[kOrder + b0] * wv[2 * kOrder + c0];
+        const int x0 = bases >> 20;
 #pragma unroll
-            for (int a0 = 0; a0 < kOrder; a0++) {
-                int x = x0 - a0;
-                x += x < 0 ? K0 : 0;
-                atomicAdd(G + ((size_t)x * K1 + y) * K2 + z, __float2int_rn(wv[a0] * wyz));
-            }
+        for (int a0 = 0; a0 < kOrder; a0++) {
+            int x = x0 - a0;
+            x += x < 0 ? K0 : 0;
+            atomicAdd(G + ((size_t)x * K1 + y) * K2 + z, __float2int_rn(wv[a0] * wyz));
         }
     }
 }
@@ -745,8 +754,8 @@ __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a) 
 void launch_spread(const Args& a, cudaStream_t s) {
     if (a.spread_atoms) {
         cudaMemsetAsync(a.qreal, 0, sizeof(float) * (size_t)a.n_real_total, s);
-        const int items = a.NB + 2 * a.n_mov_blocks;
-        k_spread_atoms<<<(items + kSpreadAtomWarps - 1) / kSpreadAtomWarps, kSpreadAtomWarps * 32, 0, s>>>(a);
+        const int parts = (a.NB + 2 * a.n_mov_blocks) * (kTile / kSpreadAtoms);
+        k_spread_atoms<<<(parts + kSpreadAtomWarps - 1) / kSpreadAtomWarps, kSpreadAtomWarps * 32, 0, s>>>(a);
         return;
     }
     if (a.brick_ctas <= 0) return;

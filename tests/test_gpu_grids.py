@@ -39,3 +39,16 @@ def test_grids_with_prime_factors_beyond_the_dedicated_radices(diff):
     outputs per work item, alone (23, 29, 31, 37) and after other stages (22, 26,
     33, 34, 38, 39)."""
     _check([(22, 23, 26), (31, 29, 37), (34, 39, 38), (33, 22, 22), (26, 22, 34)], diff)
+
+
+@pytest.mark.parametrize("ligand", [7, 8, 9, 33], ids=lambda n: f"ligand{n}")
+def test_default_spreading_gives_the_bricks_bits(ligand):
+    """Per-atom spreading (the default) against bricks: blocks that end one atom
+    before, at and after a warp's share of a block, and a moving block of one atom."""
+    c = S.water_ligand_box(1300 + ligand, 2.6, [ligand], [(1.3, 1.2, 1.1)], S.PME, 0.9, seed=70)
+    out = []
+    for props in ({}, {"SpreadBrick": 16}, {"SpreadByOwner": 0}):
+        b = atm.ReplicaBatch([atm.system_from_case(c)[0]], 0, props)
+        out.append(b.evaluate(c.pos, as_array=True))
+    for E, F, r in out[1:]:
+        assert np.array_equal(F, out[0][1]) and np.array_equal(r, out[0][2])
