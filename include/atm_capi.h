@@ -329,8 +329,8 @@ int atm_md_get_records(atm_md_t md, long long* steps, double* results, double* m
  * d_epsilon (n each), excluded partners as CSR (d_excl_start[n+1], d_excl,
  * both directions listed), outputs d_energy (1, kJ/mol) and d_forces (n x 3,
  * kJ/mol/nm); box = 3 host doubles (orthorhombic edges, each >= 2 cutoff).
- * It allocates nothing: its scratch (about 400 KB of fixed-point force
- * accumulators and energy partials) is a static device array that every GPU
+ * It allocates nothing: its scratch (about 800 KB of fixed-point force
+ * accumulators, FP32 positions and energy partials) is a static device array that every GPU
  * loading the library holds until exit, cleared at the start of every call.
  * The first call on a device looks up that array's address; make that first
  * call before any stream capture.  Calls that overlap on the GPU (other

@@ -52,3 +52,37 @@ def test_default_spreading_gives_the_bricks_bits(ligand):
         out.append(b.evaluate(c.pos, as_array=True))
     for E, F, r in out[1:]:
         assert np.array_equal(F, out[0][1]) and np.array_equal(r, out[0][2])
+
+
+@pytest.mark.parametrize("n,edge", [(31, 1.9), (33, 1.9), (65, 9.0), (65, 3.6), (1500, 2.5), (16384, 5.6)])
+def test_noalloc_skips_no_pair(n, edge):
+    """Tiles and steps left out hold no counted pair: one block, one particle past a
+    block, blocks mostly beyond the cutoff, a dense box and the largest count, with
+    particles outside the cell and blocks that span it, against the oracle."""
+    import ctypes as C
+
+    import torch
+    from atmmetaforce import _lib
+
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1 / 3)))
+    g = (np.arange(side) + 0.5) * (edge / side)
+    pos = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)[rng.permutation(side ** 3)[:n]]
+    pos += rng.uniform(-0.02, 0.02, (n, 3)) + edge * rng.integers(-2, 3, (n, 3))
+    q, sig, eps = rng.uniform(-0.4, 0.4, n), rng.uniform(0.15, 0.2, n), rng.uniform(0.1, 0.5, n)
+    ei = np.arange(0, n - 1, 2, dtype=np.int32)
+    zero = np.zeros(len(ei))
+    spec = S.NonbondedSpec(q, sig, eps, ei, ei + 1, zero, zero + 1.0, zero, S.CUTOFF_PERIODIC, 0.9, np.full(3, edge))
+    start = np.concatenate([[0], np.cumsum(np.arange(n) < 2 * len(ei))]).astype(np.int32)
+    flat = (np.arange(2 * len(ei)) ^ 1).astype(np.int32)
+    d = lambda a: torch.as_tensor(np.ascontiguousarray(a), device="cuda")  # noqa: E731
+    args = [d(a) for a in (pos, q, sig, eps, start, flat)]
+    e = torch.zeros(1, dtype=torch.float64, device="cuda")
+    f = torch.zeros(n, 3, dtype=torch.float64, device="cuda")
+    _lib.call("atm_rf_nonbonded_noalloc", n, *(C.c_void_p(a.data_ptr()) for a in args), (C.c_double * 3)(*spec.box), 0.9,
+              78.5, C.c_void_p(e.data_ptr()), C.c_void_p(f.data_ptr()), None)
+    torch.cuda.synchronize()
+    E, F, T = O.nonbonded(spec, pos)
+    assert abs(e.item() - E) <= 2e-6 * (sum(abs(v) for v in T.values()) + 1.0)
+    # (no pair at all in the sparsest box: both are zero)
+    assert np.sqrt(((f.cpu().numpy() - F) ** 2).sum()) <= F_TOL * np.sqrt((F ** 2).sum())
