@@ -209,23 +209,21 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
     CUDA_CHECK(cudaStreamCreateWithFlags(&s_pme_, cudaStreamNonBlocking));
     CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     CUDA_CHECK(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
-    CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork2_, cudaEventDisableTiming));
-    CUDA_CHECK(cudaEventCreateWithFlags(&ev_join2_, cudaEventDisableTiming));
     CUDA_CHECK(cudaMallocHost(&h_pos_, sizeof(double) * 3 * (size_t)n_in_));
     CUDA_CHECK(cudaMallocHost(&h_forces_, sizeof(double) * 3 * (size_t)n_in_));
     CUDA_CHECK(cudaMallocHost(&h_fnb_, sizeof(double) * 3 * (size_t)n_in_));
     CUDA_CHECK(cudaMallocHost(&h_results_, sizeof(double) * NUM_RES * (size_t)R_));
     CUDA_CHECK(cudaMallocHost(&h_matrix_, sizeof(double) * (size_t)R_ * R_));
-    // parameter block: ctl (2 ints) at 0, io (3 pointers) at 8, beta at 32, the
+    // parameter block: ctl (2 ints) at 0, io (4 pointers) at 8, beta at 40, the
     // replica table at kParamReps
     param_bytes_ = kParamReps + sizeof(RepDev) * (size_t)R_;
     CUDA_CHECK(cudaMallocHost(&h_params_, param_bytes_));
     std::memset(h_params_, 0, param_bytes_);
     h_ctl_ = reinterpret_cast<int*>(h_params_);
     h_io_ = reinterpret_cast<double**>(h_params_ + 8);
-    h_beta_ = reinterpret_cast<double*>(h_params_ + 32);
+    h_beta_ = reinterpret_cast<double*>(h_params_ + 40);
     h_reps_ = reinterpret_cast<RepDev*>(h_params_ + kParamReps);
-    h_io_[0] = h_io_[1] = h_io_[2] = nullptr;
+    for (int k = 0; k < 4; k++) h_io_[k] = nullptr;
     CUDA_CHECK(cudaMalloc(&d_counts_, 2 * sizeof(long long)));
     CUDA_CHECK(cudaMemset(d_counts_, 0, 2 * sizeof(long long)));
     h_ctl_[0] = 1;
@@ -259,17 +257,14 @@ Engine::~Engine() {
     cudaFreeHost(h_status_);
     if (ev_fork_) cudaEventDestroy(ev_fork_);
     if (ev_join_) cudaEventDestroy(ev_join_);
-    if (ev_fork2_) cudaEventDestroy(ev_fork2_);
-    if (ev_join2_) cudaEventDestroy(ev_join2_);
     if (s_main_) cudaStreamDestroy(s_main_);
     if (s_pme_) cudaStreamDestroy(s_pme_);
 }
 
 void Engine::destroy_graphs() {
-    if (graph_host_) cudaGraphExecDestroy(graph_host_);
     if (graph_dev_) cudaGraphExecDestroy(graph_dev_);
     if (graph_res_) cudaGraphExecDestroy(graph_res_);
-    graph_host_ = graph_dev_ = graph_res_ = nullptr;
+    graph_dev_ = graph_res_ = nullptr;
 }
 
 void Engine::set_positions(int r, const double* pos) {
@@ -1000,8 +995,8 @@ std::string Engine::autotune(int trials, bool use_cache) {
                 const int t = sh.first;
                 const bool fu = sh.second;
                 apply_tuning(t, b, s != 0, fu);
-                run(true, nullptr, nullptr);   // uploads the staged positions (buffers may be new)
-                run(false, nullptr, nullptr);  // device graph capture + one warm evaluation
+                run(nullptr, nullptr, h_pos_);  // uploads the staged positions (buffers may be new)
+                run(nullptr, nullptr);          // device graph capture + one warm evaluation
                 CUDA_CHECK(cudaEventRecord(e0, s_main_));
                 for (int k = 0; k < trials; k++) CUDA_CHECK(cudaGraphLaunch(graph_dev_, s_main_));
                 CUDA_CHECK(cudaEventRecord(e1, s_main_));
@@ -1085,6 +1080,7 @@ void Engine::alloc_device() {
     a.cutoffd = cutoff_;
     d_params_ = dalloc<char>(d_allocs_, param_bytes_);
     CUDA_CHECK(cudaMemset(d_params_, 0, param_bytes_));
+    h_params_sent_.clear();
     a.reps = reinterpret_cast<RepDev*>(d_params_ + kParamReps);
     a.pos_in = dalloc<double>(d_allocs_, 3 * (size_t)n_in_);
     {
@@ -1096,7 +1092,6 @@ void Engine::alloc_device() {
     a.slot_of = dupload(d_allocs_, slot_of_);
     a.f_out = dalloc<double>(d_allocs_, 3 * (size_t)n_in_);
     a.io = reinterpret_cast<double**>(d_params_ + 8);
-    a.f_nb = dalloc<double>(d_allocs_, 3 * (size_t)n_in_);
     a.orig = dupload(d_allocs_, orig_);
     a.qs = dupload(d_allocs_, qs_);
     a.lj = dupload(d_allocs_, lj_);
@@ -1105,6 +1100,7 @@ void Engine::alloc_device() {
     a.posq2 = full_ ? dalloc<float4>(d_allocs_, NA_) : nullptr;
     a.posq_ref = dalloc<float4>(d_allocs_, NA_);
     a.rep_hmax = dalloc<unsigned>(d_allocs_, R_);
+    CUDA_CHECK(cudaMemset(a.rep_hmax, 0, sizeof(unsigned) * (size_t)R_));
     a.list_counts = d_counts_;
     a.list_ctl = reinterpret_cast<int*>(d_params_);
     force_build_ = true;  // new buffers hold no lists
@@ -1165,7 +1161,7 @@ void Engine::alloc_device() {
         a.spread_owner = spread_owner_ || spread_atoms_ ? 1 : 0;
         a.spread_atoms = spread_atoms_ ? 1 : 0;
         a.brick_cta_rep = dupload(d_allocs_, brick_cta_rep_);
-        a.qreal = dalloc<float>(d_allocs_, n_real_);
+        a.qreal = dalloc<float>(d_allocs_, (n_real_ + 3) & ~3LL);  // zeroed in whole float4s
         a.qcplx = dalloc<float2>(d_allocs_, n_cplx_);
         a.moduli = dupload(d_allocs_, moduli_);
         a.use_fft = use_fft_ ? 1 : 0;
@@ -1207,8 +1203,10 @@ void Engine::alloc_device() {
     }
     a.results = dalloc<double>(d_allocs_, (size_t)R_ * NUM_RES);
     a.matrix = dalloc<double>(d_allocs_, (size_t)R_ * R_);
-    a.beta = reinterpret_cast<double*>(d_params_ + 32);
+    a.beta = reinterpret_cast<double*>(d_params_ + 40);
     CUDA_CHECK(cudaMemset(a.status, 0, sizeof(Status)));
+    CUDA_CHECK(cudaHostGetDevicePointer((void**)&a.h_status, h_status_, 0));
+    a.h_results = a.h_matrix = nullptr;
 }
 
 void Engine::update_rep_table() {
@@ -1219,8 +1217,11 @@ void Engine::update_rep_table() {
         for (int k = 0; k < NUM_GLOBALS; k++) rd.params[k] = s.params[k];
         rd.e_disp = s.dispersion && periodic_ ? dispersion_coefficient(s) / (s.box[0] * s.box[1] * s.box[2]) : 0.0;
     }
-    std::memcpy(h_reps_, rep_host_.data(), sizeof(RepDev) * (size_t)R_);
-    *h_beta_ = beta_;
+    if (std::memcmp(h_reps_, rep_host_.data(), sizeof(RepDev) * (size_t)R_) != 0 || *h_beta_ != beta_) {
+        settle_params();
+        std::memcpy(h_reps_, rep_host_.data(), sizeof(RepDev) * (size_t)R_);
+        *h_beta_ = beta_;
+    }
     // the finder's variant (orthorhombic or triclinic) is part of the recorded graphs
     int tric = 0;
     for (int r = 0; r < R_; r++) tric |= rep_host_[r].tric;
@@ -1242,26 +1243,36 @@ int Engine::tile_dynamic() const {
 }
 
 int Engine::launches_per_eval() const {
-    // prepare, decide, find and tiles (or the fused kernel), exceptions, finalize
-    // (with the row sums), output, matrix (+ PME kernels)
-    int n = tune_fused_ ? 7 : 8;
+    // prepare, find and tiles (or the fused kernel), finalize (with the row sums),
+    // output (with the matrix), the exceptions unless the spreading carries them
+    int n = tune_fused_ ? 4 : 5;
+    if (A_.exc_ctas > 0 && !spread_atoms_) n++;
     // spread, gather (moving atoms included) and the transforms: three of ours
     // (zy, x + convolution, inverse yz), or the convolution between library ones
     if (method_ == NonbondedForce::PME) n += use_fft_ ? 5 : 3;
     return n;
 }
 
-void Engine::record(cudaStream_t st, int mode) {
-    const Args& a = A_;
-    const bool host_io = mode == 1;
-    if (host_io) {
-        CUDA_CHECK(cudaMemcpyAsync((void*)a.pos_in, h_pos_, sizeof(double) * 3 * (size_t)n_in_,
-                                   cudaMemcpyHostToDevice, st));
-    }
+// A transfer of the parameter block that nothing has waited for still reads it.
+void Engine::settle_params() {
+    if (!params_pending_) return;
+    CUDA_CHECK(cudaStreamSynchronize(params_stream_));
+    params_pending_ = false;
+}
+
+void Engine::upload_params(cudaStream_t st) {
+    if (h_params_sent_.size() == param_bytes_ && std::memcmp(h_params_sent_.data(), h_params_, param_bytes_) == 0) return;
     CUDA_CHECK(cudaMemcpyAsync(d_params_, h_params_, param_bytes_, cudaMemcpyHostToDevice, st));
-    CUDA_CHECK(cudaMemsetAsync(a.rep_hmax, 0, sizeof(unsigned) * (size_t)R_, st));
+    h_params_sent_.assign(h_params_, h_params_ + param_bytes_);
+    params_stream_ = st;
+    params_pending_ = true;
+}
+
+// One evaluation: kernels only (the parameter block is uploaded before the graph when
+// it changed, the grids are zeroed by k_prepare and the host's copies written by the
+// last kernels).
+void Engine::record(cudaStream_t st, const Args& a) {
     launch_prepare(a, st);
-    launch_decide(a, st);
     bool pme = method_ == NonbondedForce::PME;
     if (pme) {
         // the PME chain on its own stream (overlapping the pair tiles) or in line,
@@ -1273,8 +1284,8 @@ void Engine::record(cudaStream_t st, int mode) {
         }
         // the exceptions need neither lists nor grids: they go first on this
         // stream, beside the list building
-        launch_exceptions(a, ps);
-        launch_spread(a, ps);
+        if (!a.spread_atoms) launch_exceptions(a, ps);
+        launch_spread(a, ps, true);
         pme_transforms(ps);
         launch_gather(a, ps);
         if (tune_pme_stream_) CUDA_CHECK(cudaEventRecord(ev_join_, s_pme_));
@@ -1288,32 +1299,7 @@ void Engine::record(cudaStream_t st, int mode) {
     if (!pme) launch_exceptions(a, st);
     if (pme && tune_pme_stream_) CUDA_CHECK(cudaStreamWaitEvent(st, ev_join_, 0));
     launch_finalize(a, st);
-    if (pme && tune_pme_stream_) {
-        // the R x R matrix beside the force output
-        CUDA_CHECK(cudaEventRecord(ev_fork2_, st));
-        CUDA_CHECK(cudaStreamWaitEvent(s_pme_, ev_fork2_, 0));
-        launch_matrix(a, s_pme_);
-        CUDA_CHECK(cudaEventRecord(ev_join2_, s_pme_));
-        launch_output(a, st);
-        CUDA_CHECK(cudaStreamWaitEvent(st, ev_join2_, 0));
-    } else {
-        launch_output(a, st);
-        launch_matrix(a, st);
-    }
-    // host flavours: the result records and the R x R matrix (a few KB) end the
-    // evaluation in page-locked host memory, so that a host caller needs no copy after it
-    if (mode != 0) {
-        CUDA_CHECK(cudaMemcpyAsync(h_results_, a.results, sizeof(double) * NUM_RES * (size_t)R_,
-                                   cudaMemcpyDeviceToHost, st));
-        CUDA_CHECK(cudaMemcpyAsync(h_matrix_, a.matrix, sizeof(double) * (size_t)R_ * R_, cudaMemcpyDeviceToHost,
-                                   st));
-    }
-    if (host_io) {
-        CUDA_CHECK(cudaMemcpyAsync(h_forces_, a.f_out, sizeof(double) * 3 * (size_t)n_in_, cudaMemcpyDeviceToHost,
-                                   st));
-        CUDA_CHECK(cudaMemcpyAsync(h_fnb_, a.f_nb, sizeof(double) * 3 * (size_t)n_in_, cudaMemcpyDeviceToHost, st));
-    }
-    CUDA_CHECK(cudaMemcpyAsync(h_status_, a.status, sizeof(Status), cudaMemcpyDeviceToHost, st));
+    launch_output(a, st);
 }
 
 // Charge grids -> potential grids: the hand-written transforms with the
@@ -1361,13 +1347,13 @@ bool Engine::check_status_and_grow() {
     return true;
 }
 
-void Engine::run(bool host_io, cudaStream_t user, const double* d_pos, const double* h_pos_pinned,
-                 bool host_results) {
+void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos_pinned, bool host_results) {
     CUDA_CHECK(cudaSetDevice(dev_));
     if (!layout_ready_) {
         build_layout();
         alloc_device();
     }
+    settle_params();
     for (int attempt = 0; attempt < 4; attempt++) {
         update_rep_table();
         update_influence(user ? user : s_main_);
@@ -1376,6 +1362,12 @@ void Engine::run(bool host_io, cudaStream_t user, const double* d_pos, const dou
         h_ctl_[0] = (force_build_ || skin_ <= 0.0) ? 1 : 0;
         force_build_ = false;
         cudaStream_t st = user ? user : s_main_;
+        upload_params(st);
+        Args a = A_;
+        if (profiling_ || h_pos_pinned || host_results) {
+            CUDA_CHECK(cudaHostGetDevicePointer((void**)&a.h_results, h_results_, 0));
+            CUDA_CHECK(cudaHostGetDevicePointer((void**)&a.h_matrix, h_matrix_, 0));
+        }
         if (d_pos && d_pos != h_io_[0])  // (positions the graph reads in place need no copy)
             CUDA_CHECK(cudaMemcpyAsync((void*)A_.pos_in, d_pos, sizeof(double) * 3 * (size_t)n_in_,
                                        cudaMemcpyDeviceToDevice, st));
@@ -1393,15 +1385,8 @@ void Engine::run(bool host_io, cudaStream_t user, const double* d_pos, const dou
                 ev.push_back(e);
                 times_.push_back({name, 0.0});
             };
-            const Args& a = A_;
-            if (host_io)
-                CUDA_CHECK(cudaMemcpyAsync((void*)a.pos_in, h_pos_, sizeof(double) * 3 * (size_t)n_in_,
-                                           cudaMemcpyHostToDevice, st));
-            CUDA_CHECK(cudaMemcpyAsync(d_params_, h_params_, param_bytes_, cudaMemcpyHostToDevice, st));
-            CUDA_CHECK(cudaMemsetAsync(a.rep_hmax, 0, sizeof(unsigned) * (size_t)R_, st));
             mark("start");
             launch_prepare(a, st);
-            launch_decide(a, st);
             mark("prepare");
             if (a.fused) {
                 launch_find_tiles(a, st);
@@ -1425,19 +1410,6 @@ void Engine::run(bool host_io, cudaStream_t user, const double* d_pos, const dou
             mark("finalize");
             launch_output(a, st);
             mark("output");
-            launch_matrix(a, st);
-            mark("matrix");
-            if (host_io) {
-                CUDA_CHECK(cudaMemcpyAsync(h_results_, a.results, sizeof(double) * NUM_RES * (size_t)R_,
-                                           cudaMemcpyDeviceToHost, st));
-                CUDA_CHECK(cudaMemcpyAsync(h_forces_, a.f_out, sizeof(double) * 3 * (size_t)n_in_,
-                                           cudaMemcpyDeviceToHost, st));
-                CUDA_CHECK(cudaMemcpyAsync(h_fnb_, a.f_nb, sizeof(double) * 3 * (size_t)n_in_,
-                                           cudaMemcpyDeviceToHost, st));
-                CUDA_CHECK(cudaMemcpyAsync(h_matrix_, a.matrix, sizeof(double) * (size_t)R_ * R_,
-                                           cudaMemcpyDeviceToHost, st));
-            }
-            CUDA_CHECK(cudaMemcpyAsync(h_status_, a.status, sizeof(Status), cudaMemcpyDeviceToHost, st));
             CUDA_CHECK(cudaStreamSynchronize(st));
             for (size_t k = 1; k < ev.size(); k++) {
                 float ms = 0;
@@ -1447,13 +1419,12 @@ void Engine::run(bool host_io, cudaStream_t user, const double* d_pos, const dou
             for (auto e : ev) cudaEventDestroy(e);
             times_.erase(times_.begin());
         } else {
-            const int mode = host_io ? 1 : ((h_pos_pinned || host_results) ? 2 : 0);
-            cudaGraphExec_t& gx = mode == 1 ? graph_host_ : (mode == 2 ? graph_res_ : graph_dev_);
+            cudaGraphExec_t& gx = a.h_results ? graph_res_ : graph_dev_;
             if (!gx) {
                 cudaGraph_t g;
                 CUDA_CHECK(cudaStreamBeginCapture(s_main_, cudaStreamCaptureModeThreadLocal));
                 try {
-                    record(s_main_, mode);
+                    record(s_main_, a);
                 } catch (...) {
                     cudaStreamEndCapture(s_main_, &g);
                     throw;
@@ -1465,6 +1436,7 @@ void Engine::run(bool host_io, cudaStream_t user, const double* d_pos, const dou
             CUDA_CHECK(cudaGraphLaunch(gx, st));
             CUDA_CHECK(cudaStreamSynchronize(st));
         }
+        params_pending_ = false;
         if (!check_status_and_grow()) {
             // the evaluation has run: later ones (launch_device) leave the build
             // to the device unless there is no skin
@@ -1523,44 +1495,29 @@ void Engine::evaluate(double* energies, double* forces, double* forces_nb, doubl
 void Engine::evaluate_host(const double* pos, double* energies, double* forces, double* forces_nb, double* results,
                            double* matrix) {
     CUDA_CHECK(cudaSetDevice(dev_));
+    settle_params();
     const size_t bytes = sizeof(double) * 3 * (size_t)n_in_;
     const bool pin_in = pos && is_pinned(pos);
     // the layout and the profiling path read the staging copy
     if (pos && (!pin_in || !layout_ready_ || profiling_)) par_memcpy(h_pos_, pos, bytes);
-    if (profiling_) {
-        run(true, nullptr, nullptr);
-    } else {
-        // positions straight from a pinned caller buffer, else from the pinned
-        // staging copy; forces written by the output kernel straight into a
-        // page-locked caller buffer over the host link (no copy after the graph)
-        double* zc = forces ? host_mapped(forces) : nullptr;
-        h_io_[1] = zc;
-        try {
-            run(false, s_main_, nullptr, pin_in ? pos : h_pos_);
-        } catch (...) {
-            h_io_[1] = nullptr;
-            throw;
-        }
-        h_io_[1] = nullptr;  // (the graph that read it has finished)
-        const bool copy_f = forces && !zc;
-        if (copy_f || forces_nb) {
-            const bool pin_out = copy_f && is_pinned(forces);
-            cudaStream_t st = s_main_;
-            if (copy_f)
-                CUDA_CHECK(cudaMemcpyAsync(pin_out ? forces : h_forces_, A_.f_out, bytes, cudaMemcpyDeviceToHost, st));
-            if (forces_nb) CUDA_CHECK(cudaMemcpyAsync(h_fnb_, A_.f_nb, bytes, cudaMemcpyDeviceToHost, st));
-            CUDA_CHECK(cudaStreamSynchronize(st));
-            if (copy_f && !pin_out) par_memcpy(forces, h_forces_, bytes);
-            if (forces_nb) par_memcpy(forces_nb, h_fnb_, bytes);
-        }
-        forces = nullptr;
-        forces_nb = nullptr;
+    // positions straight from a pinned caller buffer, else from the pinned staging
+    // copy; forces written by the output kernel over the host link, straight into a
+    // page-locked caller buffer or else into the pinned staging copies
+    double* const zc = forces ? host_mapped(forces) : nullptr;
+    h_io_[1] = zc ? zc : (forces ? host_mapped(h_forces_) : nullptr);
+    h_io_[3] = forces_nb ? host_mapped(h_fnb_) : nullptr;
+    try {
+        run(s_main_, nullptr, pin_in && !profiling_ ? pos : h_pos_);
+    } catch (...) {
+        h_io_[1] = h_io_[3] = nullptr;
+        throw;
     }
+    h_io_[1] = h_io_[3] = nullptr;  // (the graph that read them has finished)
+    if (forces && !zc) par_memcpy(forces, h_forces_, bytes);
+    if (forces_nb) par_memcpy(forces_nb, h_fnb_, bytes);
     for (int r = 0; r < R_; r++) {
         if (energies) energies[r] = h_results_[(size_t)r * NUM_RES + RES_ENERGY];
     }
-    if (forces) std::memcpy(forces, h_forces_, bytes);
-    if (forces_nb) std::memcpy(forces_nb, h_fnb_, bytes);
     if (results) std::memcpy(results, h_results_, sizeof(double) * NUM_RES * (size_t)R_);
     if (matrix) std::memcpy(matrix, h_matrix_, sizeof(double) * (size_t)R_ * R_);
 }
@@ -1574,7 +1531,7 @@ void Engine::run_device(const double* d_pos, cudaStream_t stream) {
         build_layout();
         alloc_device();
     }
-    run(false, stream, d_pos);
+    run(stream, d_pos);
 }
 
 void Engine::launch_device(const double* d_pos, cudaStream_t stream) {
@@ -1596,6 +1553,7 @@ void Engine::launch_device(const double* d_pos, cudaStream_t stream) {
     if (d_pos != h_io_[0])
         CUDA_CHECK(cudaMemcpyAsync((void*)A_.pos_in, d_pos, sizeof(double) * 3 * (size_t)n_in_,
                                    cudaMemcpyDeviceToDevice, stream));
+    upload_params(stream);
     CUDA_CHECK(cudaGraphLaunch(graph_dev_, stream));
 }
 
@@ -1632,6 +1590,7 @@ void Engine::evaluate_device(const double* d_pos, double* d_forces, double* d_re
     // the evaluation reads the caller's positions in place and writes the caller's
     // forces and result records itself (no copies before or after the graph); the
     // records and matrix also end in page-locked host memory
+    settle_params();
     double* const keep = h_io_[0];
     h_io_[0] = const_cast<double*>(d_pos);
     h_io_[1] = d_forces;
@@ -1645,7 +1604,7 @@ void Engine::evaluate_device(const double* d_pos, double* d_forces, double* d_re
             build_layout();
             alloc_device();
         }
-        run(false, stream, d_pos, nullptr, true);  // synchronises
+        run(stream, d_pos, nullptr, true);  // synchronises
     } catch (...) {
         h_io_[0] = keep;
         h_io_[1] = h_io_[2] = nullptr;

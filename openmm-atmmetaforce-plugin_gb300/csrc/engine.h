@@ -155,16 +155,14 @@ private:
     void upload_static();
     void fill_args();
     void update_rep_table();
-    // graph flavours: 0 device buffers only (MD, torch), 1 host staging copies of
-    // positions, forces and results, 2 results and matrix to the host (positions
-    // copied in before the launch, forces to a page-locked caller buffer or copied
-    // after it)
-    void record(cudaStream_t main, int mode);
+    void record(cudaStream_t main, const Args& a);
     void pme_transforms(cudaStream_t st, const std::function<void(const char*)>& mark = nullptr);
-    // host_results: the result records and matrix end in h_results_ / h_matrix_ (graph
-    // flavour 2) without host positions
-    void run(bool host_io, cudaStream_t user, const double* d_pos, const double* h_pos_pinned = nullptr,
-             bool host_results = false);
+    // The device mirror of the parameter block, brought up to date on the stream.
+    void upload_params(cudaStream_t st);
+    void settle_params();
+    // host_results (implied by h_pos_pinned): the result records and the matrix also end
+    // in h_results_ / h_matrix_
+    void run(cudaStream_t user, const double* d_pos, const double* h_pos_pinned = nullptr, bool host_results = false);
     bool check_status_and_grow();
     void destroy_graphs();
 
@@ -245,17 +243,21 @@ private:
     double* h_results_ = nullptr;  // R*NUM_RES
     double* h_matrix_ = nullptr;   // R*R
     // The per-evaluation parameters in one page-locked block (list control word,
-    // caller buffers, beta, replica table), which every evaluation copies to its
-    // device mirror with one transfer; the four pointers below point into it.
+    // caller buffers, beta, replica table), copied to its device mirror with one
+    // transfer when they differ from what the mirror holds (h_params_sent_, empty:
+    // nothing yet); the four pointers below point into it.
     static constexpr size_t kParamReps = 64;  // byte offset of the replica table
     size_t param_bytes_ = 0;
     char* h_params_ = nullptr;
     char* d_params_ = nullptr;
+    std::vector<char> h_params_sent_;
+    cudaStream_t params_stream_ = nullptr;  // with a transfer that nothing has waited for
+    bool params_pending_ = false;
     RepDev* h_reps_ = nullptr;     // R
     double* h_beta_ = nullptr;
-    int* h_ctl_ = nullptr;         // list control word, copied to the device by every evaluation
-    double** h_io_ = nullptr;      // caller buffers of the next evaluations (Args::io), copied to the
-                                   // device by every evaluation: positions, forces, result records
+    int* h_ctl_ = nullptr;         // list control word
+    double** h_io_ = nullptr;      // caller buffers of the next evaluations (Args::io): positions,
+                                   // forces, result records, state-1 nonbonded forces
     Status* h_status_ = nullptr;
 
     // device buffers
@@ -264,8 +266,8 @@ private:
     std::vector<void*> d_allocs_;
 
     cudaStream_t s_main_ = nullptr, s_pme_ = nullptr;
-    cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr, ev_fork2_ = nullptr, ev_join2_ = nullptr;
-    cudaGraphExec_t graph_host_ = nullptr, graph_dev_ = nullptr, graph_res_ = nullptr;
+    cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
+    cudaGraphExec_t graph_dev_ = nullptr, graph_res_ = nullptr;  // without / with host results
     std::vector<KernelTime> times_;
 };
 

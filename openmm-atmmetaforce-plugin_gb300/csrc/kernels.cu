@@ -2,20 +2,22 @@
 //
 // Data flow of one evaluation of R replicas:
 //   prepare  : user positions (FP64) -> wrapped float4 slots, state-2 copies,
-//              block bounding boxes; zero the force accumulators
-//   find     : one warp per tile row -> compacted list of interacting 32x32 tiles
+//              block bounding boxes; zero the force accumulators and charge grids;
+//              decide whether the lists are built
+//   find     : one warp per tile row -> compacted list of interacting tiles
 //   tiles    : persistent warps over the tile list: LJ + reaction field / Ewald
 //              direct space, tile rotation by warp shuffles, fixed-point forces
-//   exceptions: exception pairs and Ewald exclusion corrections in FP64
-//   spread / convert / (cuFFT R2C) / conv / (cuFFT C2R) / gather : smooth PME
+//   spread / transforms with the convolution / gather : smooth PME; the exceptions
+//              (FP64 and FP32) and Ewald exclusion corrections beside the spreading
 //   finalize : FP64 energies, soft-core + softplus merge (ATM scalars)
-//   output   : hybrid forces F1 + s' (F2 - F1) in user order
-//   matrix   : replicas x states reduced-energy matrix
+//   output   : hybrid forces F1 + s' (F2 - F1) in user order, and the replicas x
+//              states reduced-energy matrix
 //
 // Reference semantics: inner evaluations of ATMMetaForceImpl.cpp:113,116; the
 // displacement of CopyState, platforms/common/src/kernels/atmmetaforce.cc:19-52;
 // the merge of ReferenceATMMetaForceKernels.cpp:56-113 (FP64, as the Reference
 // platform, instead of the float `sp` of CommonATMMetaForceKernels.cpp:199).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 
@@ -62,79 +64,12 @@ __device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDe
     }
 }
 
-__global__ void k_prepare(Args a) {
-    int lane = threadIdx.x & 31;
-    int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (b >= a.NB) return;
-    int s = b * kTile + lane;
-    int rep = a.block_rep[b];
-    const RepDev& R = a.reps[rep];
-    int o = a.orig[s];
-    const int nreal = __popc(__ballot_sync(FULL_MASK, o >= 0));  // padding sits at the end of a block
-    if (o < 0) o = a.orig[b * kTile];  // padding copies the block's first atom
-    const double* p = (a.io[0] ? a.io[0] : a.pos_in) + 3 * (size_t)(R.in_off + o);
-    double xd = p[0], yd = p[1], zd = p[2];
-    float x = (float)xd, y = (float)yd, z = (float)zd;
-    // a position whose reduced coordinates lie safely inside (0, 1) (by 1e-5, far
-    // beyond the FP32 estimate's error) is in the unit cell already: the FP64 wrap
-    // would subtract zero.  Others take the FP64 wrap (FP64 is 1/64 of the FP32
-    // rate on this part).
-    constexpr float kIn = 1e-5f;
-    const float ux = x * R.ibox[0], uy = y * R.ibox[1], uz = z * R.ibox[2];
-    if (!(ux >= kIn && ux <= 1.0f - kIn && uy >= kIn && uy <= 1.0f - kIn && uz >= kIn && uz <= 1.0f - kIn)) {
-        wrap3d(xd, yd, zd, R);  // FP64 wrap into the unit cell
-        x = (float)xd;
-        y = (float)yd;
-        z = (float)zd;
-    }
-    float q = a.qs[s];
-    a.posq[s] = make_float4(x, y, z, q);
-    if (a.skin_half2 > 0.f) {
-        // displacement since the last list build (minimum image: wrapping is no motion)
-        const float4 r = a.posq_ref[s];
-        float dx = x - r.x, dy = y - r.y, dz = z - r.z;
-        min_image3(dx, dy, dz, R);
-        float d2 = dx * dx + dy * dy + dz * dz;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) d2 = fmaxf(d2, __shfl_xor_sync(FULL_MASK, d2, o));
-        // non-negative floats order as their bit patterns
-        if (lane == 0) atomicMax(&a.status->disp2, __float_as_uint(d2));
-    }
-    for (int k = 0; k < 6; k++) a.F[(size_t)k * a.NA + s] = 0ull;
-    if (a.adjoint)
-        for (int k = 0; k < 3; k++) a.D[(size_t)k * a.NA + s] = 0ull;
-    warp_bbox(x, y, z, R, &a.bb_c[b], &a.bb_h[b], lane, nreal);
-    if (R.tric && lane == 0) {  // (lane 0 wrote the box)
-        const float4 h = a.bb_h[b];
-        atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));
-    }
-    if (a.full) {
-        float4 d = a.displ[s];
-        float x2 = x + d.x, y2 = y + d.y, z2 = z + d.z;
-        wrap3(x2, y2, z2, R);
-        a.posq2[s] = make_float4(x2, y2, z2, q);
-        warp_bbox(x2, y2, z2, R, &a.bb_c2[b], &a.bb_h2[b], lane, nreal);
-        if (R.tric && lane == 0) {
-            const float4 h = a.bb_h2[b];
-            atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));
-        }
-    }
-    if (b == 0 && lane == 0) a.status->next_tile = 0;
-}
-
-void launch_prepare(const Args& a, cudaStream_t s) {
-    int threads = 256;
-    int blocks = (a.NB * 32 + threads - 1) / threads;
-    k_prepare<<<blocks, threads, 0, s>>>(a);
-}
-
 // Whether this evaluation builds the lists: when forced, with no skin, or when an
 // atom has moved more than skin / 2 since the last build (then no pair within the
 // cutoff now was beyond rc + skin then).  A build resets the finder's counters.
-__global__ void k_decide(Args a) {
-    if (threadIdx.x != 0) return;
+__device__ __forceinline__ void decide_build(const Args& a) {
     Status* st = a.status;
-    const float d2 = __uint_as_float(st->disp2);
+    const float d2 = __uint_as_float(atomicExch(&st->disp2, 0u));
     const bool build = a.list_ctl[0] != 0 || !(a.skin_half2 > 0.f) || d2 > a.skin_half2;
     st->sticky |= st->overflow;
     if (build) {
@@ -143,13 +78,106 @@ __global__ void k_decide(Args a) {
         st->max_row = 0;
     }
     st->next_row = 0;  // the fused kernel walks the rows at every evaluation
+    st->next_tile = 0;
+    st->prepared = 0;
     st->rebuild = build ? 1 : 0;
-    st->disp2 = 0u;
     a.list_counts[0]++;
     if (build) a.list_counts[1]++;
 }
 
-void launch_decide(const Args& a, cudaStream_t s) { k_decide<<<1, 32, 0, s>>>(a); }
+constexpr int kPrepThreads = 256;
+
+// CTAs below nprep prepare eight blocks each; the rest zero the int32 charge grids,
+// which the spreading adds into (a memset node of its own cost the PME chain its
+// launch and its drain).  The list decision needs every displacement: the last
+// preparing CTA takes it (without a skin it needs none, and CTA 0 does).
+__global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
+    if ((int)blockIdx.x >= nprep) {
+        const long long n4 = (a.n_real_total + 3) >> 2;  // (allocated in whole float4s)
+        float4* g = reinterpret_cast<float4*>(a.qreal);
+        const long long stride = (long long)(gridDim.x - nprep) * kPrepThreads;
+        for (long long k = (long long)(blockIdx.x - nprep) * kPrepThreads + threadIdx.x; k < n4; k += stride)
+            g[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    int lane = threadIdx.x & 31;
+    int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b < a.NB) {
+        int s = b * kTile + lane;
+        int rep = a.block_rep[b];
+        const RepDev& R = a.reps[rep];
+        int o = a.orig[s];
+        const int nreal = __popc(__ballot_sync(FULL_MASK, o >= 0));  // padding sits at the end of a block
+        if (o < 0) o = a.orig[b * kTile];  // padding copies the block's first atom
+        const double* p = (a.io[0] ? a.io[0] : a.pos_in) + 3 * (size_t)(R.in_off + o);
+        double xd = p[0], yd = p[1], zd = p[2];
+        float x = (float)xd, y = (float)yd, z = (float)zd;
+        // a position whose reduced coordinates lie safely inside (0, 1) (by 1e-5, far
+        // beyond the FP32 estimate's error) is in the unit cell already: the FP64 wrap
+        // would subtract zero.  Others take the FP64 wrap (FP64 is 1/64 of the FP32
+        // rate on this part).
+        constexpr float kIn = 1e-5f;
+        const float ux = x * R.ibox[0], uy = y * R.ibox[1], uz = z * R.ibox[2];
+        if (!(ux >= kIn && ux <= 1.0f - kIn && uy >= kIn && uy <= 1.0f - kIn && uz >= kIn && uz <= 1.0f - kIn)) {
+            wrap3d(xd, yd, zd, R);  // FP64 wrap into the unit cell
+            x = (float)xd;
+            y = (float)yd;
+            z = (float)zd;
+        }
+        float q = a.qs[s];
+        a.posq[s] = make_float4(x, y, z, q);
+        if (a.skin_half2 > 0.f) {
+            // displacement since the last list build (minimum image: wrapping is no motion)
+            const float4 r = a.posq_ref[s];
+            float dx = x - r.x, dy = y - r.y, dz = z - r.z;
+            min_image3(dx, dy, dz, R);
+            float d2 = dx * dx + dy * dy + dz * dz;
+    #pragma unroll
+            for (int o = 16; o > 0; o >>= 1) d2 = fmaxf(d2, __shfl_xor_sync(FULL_MASK, d2, o));
+            // non-negative floats order as their bit patterns
+            if (lane == 0) atomicMax(&a.status->disp2, __float_as_uint(d2));
+        }
+        for (int k = 0; k < 6; k++) a.F[(size_t)k * a.NA + s] = 0ull;
+        if (a.adjoint)
+            for (int k = 0; k < 3; k++) a.D[(size_t)k * a.NA + s] = 0ull;
+        warp_bbox(x, y, z, R, &a.bb_c[b], &a.bb_h[b], lane, nreal);
+        if (R.tric && lane == 0) {  // (lane 0 wrote the box)
+            const float4 h = a.bb_h[b];
+            atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));
+        }
+        if (a.full) {
+            float4 d = a.displ[s];
+            float x2 = x + d.x, y2 = y + d.y, z2 = z + d.z;
+            wrap3(x2, y2, z2, R);
+            a.posq2[s] = make_float4(x2, y2, z2, q);
+            warp_bbox(x2, y2, z2, R, &a.bb_c2[b], &a.bb_h2[b], lane, nreal);
+            if (R.tric && lane == 0) {
+                const float4 h = a.bb_h2[b];
+                atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));
+            }
+        }
+    }
+    if (a.skin_half2 > 0.f) {
+        __syncthreads();  // this CTA's maxima precede its count
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(&a.status->prepared, 1) == nprep - 1) {
+                __threadfence();
+                decide_build(a);
+            }
+        }
+    } else if (blockIdx.x == 0 && threadIdx.x == 0) {
+        decide_build(a);
+    }
+}
+
+void launch_prepare(const Args& a, cudaStream_t s) {
+    const int nprep = (a.NB * 32 + kPrepThreads - 1) / kPrepThreads;
+    long long nzero = 0;
+    if (a.spread_owner)  // eight float4 per thread
+        nzero = std::min<long long>((a.n_real_total + 32 * kPrepThreads - 1) / (32 * kPrepThreads), 4096);
+    k_prepare<<<nprep + (int)nzero, kPrepThreads, 0, s>>>(a, nprep);
+}
 
 // ---------------------------------------------------------------------------
 // find: one warp per row; bounding-box test of block I against candidates J
@@ -250,9 +278,11 @@ __device__ __forceinline__ float exc_term_f(const Args& a, const RepDev& R, cons
     return e;
 }
 
-__global__ void __launch_bounds__(256) k_exceptions(Args a) {
+constexpr int kExcThreads = 256;
+
+// The exceptions of CTA c (kExcThreads threads).
+__device__ __forceinline__ void exceptions_cta(const Args& a, int c) {
     __shared__ double red[3][8];
-    int c = blockIdx.x;
     int e = a.exc_cta_first[c] + threadIdx.x;
     float E1f = 0.0f;  // same-class pairs (FP32 terms, summed in FP32 within a warp)
     double E1 = 0.0, E2 = 0.0, DE = 0.0;
@@ -331,8 +361,10 @@ __global__ void __launch_bounds__(256) k_exceptions(Args a) {
     }
 }
 
+__global__ void __launch_bounds__(kExcThreads) k_exceptions(Args a) { exceptions_cta(a, blockIdx.x); }
+
 void launch_exceptions(const Args& a, cudaStream_t s) {
-    if (a.exc_ctas > 0) k_exceptions<<<a.exc_ctas, 256, 0, s>>>(a);
+    if (a.exc_ctas > 0) k_exceptions<<<a.exc_ctas, kExcThreads, 0, s>>>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -682,11 +714,20 @@ __global__ void __launch_bounds__(kBrickThreads) k_spread(Args a) {
 constexpr int kSpreadAtomWarps = 8;
 constexpr int kSpreadAtoms = 8;
 
-__global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a) {
+//
+// The first nexc CTAs evaluate the exceptions, which the PME chain would otherwise
+// wait for (5 of its 60 us on one 23,558-atom box).
+static_assert(kExcThreads == kSpreadAtomWarps * 32, "exceptions and spreading share a launch");
+
+__global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a, int nexc) {
     __shared__ float s_st[kSpreadAtomWarps][kSpreadAtoms * kStencilWords];
+    if ((int)blockIdx.x < nexc) {
+        exceptions_cta(a, blockIdx.x);
+        return;
+    }
     constexpr int kParts = kTile / kSpreadAtoms;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int part_item = blockIdx.x * kSpreadAtomWarps + w;
+    const int part_item = (blockIdx.x - nexc) * kSpreadAtomWarps + w;
     const int item = part_item / kParts, part = part_item - item * kParts;
     if (item >= a.NB + 2 * a.n_mov_blocks) return;
     int blk, code;  // 0: grid 0 at x; 1: grid 1, -q at x; 3: grid 1, +q at x + d
@@ -751,16 +792,15 @@ __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a) 
     }
 }
 
-void launch_spread(const Args& a, cudaStream_t s) {
+// (the int32 grids were zeroed by k_prepare)
+void launch_spread(const Args& a, cudaStream_t s, bool with_exceptions) {
     if (a.spread_atoms) {
-        cudaMemsetAsync(a.qreal, 0, sizeof(float) * (size_t)a.n_real_total, s);
         const int parts = (a.NB + 2 * a.n_mov_blocks) * (kTile / kSpreadAtoms);
-        k_spread_atoms<<<(parts + kSpreadAtomWarps - 1) / kSpreadAtomWarps, kSpreadAtomWarps * 32, 0, s>>>(a);
+        const int nexc = with_exceptions ? a.exc_ctas : 0;
+        k_spread_atoms<<<nexc + (parts + kSpreadAtomWarps - 1) / kSpreadAtomWarps, kSpreadAtomWarps * 32, 0, s>>>(a, nexc);
         return;
     }
     if (a.brick_ctas <= 0) return;
-    // owner mode adds every brick into the grids: they start at zero
-    if (a.spread_owner) cudaMemsetAsync(a.qreal, 0, sizeof(float) * (size_t)a.n_real_total, s);
     const int bytes = spread_smem_bytes(a.brick_smem);
     // opt in to more than 48 KB of dynamic shared memory (per device; this runs
     // when the evaluation graph is recorded, not at every evaluation)
@@ -1228,6 +1268,9 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(Args a) {
         out[RES_STATUS] = (double)a.status->overflow;
         if (a.io[2])
             for (int k = 0; k < NUM_RES; k++) a.io[2][(size_t)r * NUM_RES + k] = out[k];
+        if (a.h_results)
+            for (int k = 0; k < NUM_RES; k++) a.h_results[(size_t)r * NUM_RES + k] = out[k];
+        a.rep_hmax[r] = 0u;  // ready for the next evaluation (the finder has read it)
     }
 }
 
@@ -1242,10 +1285,31 @@ void launch_finalize(const Args& a, cudaStream_t s) {
 // without a separate copy.
 constexpr int kOutThreads = 256;
 
-__global__ void __launch_bounds__(kOutThreads) k_output(Args a) {
+// replicas x states energy matrix: beta * (e0(r; dir_s) + W_s(usc_s(u(r; dir_s)))), entry idx
+__device__ __forceinline__ void matrix_entry(const Args& a, int idx) {
+    int r = idx / a.R, s = idx % a.R;
+    const double* res = a.results + (size_t)r * NUM_RES;
+    double out[NUM_RES];
+    bool v = a.reps[r].var_nb;
+    atm_merge(v ? res[RES_E1] : 0.0, v ? res[RES_E2] : 0.0, a.reps[s].params, out);
+    const double e = *a.beta * out[RES_ENERGY];
+    a.matrix[idx] = e;
+    if (a.h_matrix) a.h_matrix[idx] = e;
+}
+
+// The first nmat CTAs compute the matrix (a chain of FP64 functions about as long as
+// the whole force output, so beside it) and hand the status to the host.
+__global__ void __launch_bounds__(kOutThreads) k_output(Args a, int nmat) {
     __shared__ double s_f[kOutThreads / 32][96];
-    const int g = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if ((int)blockIdx.x < nmat) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.h_status = *a.status;
+        const int idx = blockIdx.x * kOutThreads + threadIdx.x;
+        if (idx < a.R * a.R) matrix_entry(a, idx);
+        return;
+    }
+    const int g = (blockIdx.x - nmat) * kOutThreads + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double* const fo = a.io[1] ? a.io[1] : a.f_out;
+    double* const fnb = a.io[3];
     double f[3] = {0.0, 0.0, 0.0};
     if (g < a.n_in) {
         const int s = a.slot_of[g];
@@ -1268,7 +1332,7 @@ __global__ void __launch_bounds__(kOutThreads) k_output(Args a) {
             const unsigned long long lo = (unsigned long long)d * (unsigned long long)w32;
             const long long v = f1 + (long long)(((unsigned long long)hi << 32) | (lo >> 32));
             f[k] = R.var_nb ? fix_scaled(v) : 0.0;
-            if (a.f_nb) a.f_nb[3 * (size_t)g + k] = fix_scaled(f1);
+            if (fnb) fnb[3 * (size_t)g + k] = fix_scaled(f1);
         }
     }
     const int g0 = g - lane;  // the warp's first atom
@@ -1290,24 +1354,8 @@ __global__ void __launch_bounds__(kOutThreads) k_output(Args a) {
 }
 
 void launch_output(const Args& a, cudaStream_t s) {
-    k_output<<<(a.n_in + kOutThreads - 1) / kOutThreads, kOutThreads, 0, s>>>(a);
-}
-
-// replicas x states energy matrix: beta * (e0(r; dir_s) + W_s(usc_s(u(r; dir_s))))
-__global__ void k_matrix(Args a) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= a.R * a.R) return;
-    int r = idx / a.R, s = idx % a.R;
-    const double* res = a.results + (size_t)r * NUM_RES;
-    double out[NUM_RES];
-    bool v = a.reps[r].var_nb;
-    atm_merge(v ? res[RES_E1] : 0.0, v ? res[RES_E2] : 0.0, a.reps[s].params, out);
-    a.matrix[idx] = *a.beta * out[RES_ENERGY];
-}
-
-void launch_matrix(const Args& a, cudaStream_t s) {
-    int n = a.R * a.R;
-    k_matrix<<<(n + 127) / 128, 128, 0, s>>>(a);
+    const int nmat = (a.R * a.R + kOutThreads - 1) / kOutThreads;
+    k_output<<<nmat + (a.n_in + kOutThreads - 1) / kOutThreads, kOutThreads, 0, s>>>(a, nmat);
 }
 
 // Backward pass of L = sum_r g_r W_r from the last (adjoint) evaluation.  With

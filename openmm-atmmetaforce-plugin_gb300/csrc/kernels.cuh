@@ -200,6 +200,7 @@ struct Status {
     int rebuild;      // 1: the lists are built in this evaluation
     unsigned disp2;   // largest squared displacement since the last build (float bits)
     int sticky;       // overflow bits of every build since the host last cleared them
+    int prepared;     // CTAs of k_prepare done (list skin > 0; the last one decides and resets it)
 };
 
 // Arguments shared by the kernels of one engine (passed by value).
@@ -227,12 +228,12 @@ struct Args {
     const double* displ_in;   // 3*n_in
     const int* slot_of;       // n_in
     double* f_out;            // 3*n_in (ATM force)
-    double* const* io;        // device cells, copied from the host by every evaluation: io[0] the
+    double* const* io;        // device cells, copied from the host when they change: io[0] the
                               // caller's device positions, read in place of pos_in; io[1] the
                               // caller's force buffer (device, or page-locked host memory
                               // written over the host link) in place of f_out; io[2] the
-                              // caller's device result records (a copy of results); null: unused
-    double* f_nb;             // 3*n_in (state-1 nonbonded force) or null
+                              // caller's device result records (a copy of results); io[3] the
+                              // state-1 nonbonded force (3*n_in); null: unused
     // slot arrays
     const int* orig;          // NA: user index within the replica, -1 for padding
     const float* qs;          // NA: charge * sqrt(1/(4 pi eps0))
@@ -319,15 +320,20 @@ struct Args {
     double* results;          // R * NUM_RES
     double* matrix;           // R * R
     const double* beta;       // device scalar
+    // page-locked host memory the last kernels write over the host link (no copies
+    // after them): the status always, results and matrix where a host caller reads them
+    Status* h_status;
+    double* h_results;        // or null
+    double* h_matrix;         // or null
 };
 
 void launch_prepare(const Args& a, cudaStream_t s);
-void launch_decide(const Args& a, cudaStream_t s);
 void launch_find(const Args& a, cudaStream_t s);
 void launch_tiles(const Args& a, int grid, cudaStream_t s);
 void launch_find_tiles(const Args& a, cudaStream_t s);
 void launch_exceptions(const Args& a, cudaStream_t s);
-void launch_spread(const Args& a, cudaStream_t s);
+// with_exceptions: the exceptions in the same launch (per-atom spreading only)
+void launch_spread(const Args& a, cudaStream_t s, bool with_exceptions = false);
 void launch_conv(const Args& a, cudaStream_t s);
 void launch_gather(const Args& a, cudaStream_t s);
 void launch_fft_forward(const Args& a, cudaStream_t s);
@@ -341,7 +347,6 @@ void launch_influence(float* G, const float* moduli, const int* mod_off, const i
 int fft_conv_smem_bytes(int K0, int nz);
 void launch_finalize(const Args& a, cudaStream_t s);
 void launch_output(const Args& a, cudaStream_t s);
-void launch_matrix(const Args& a, cudaStream_t s);
 // Gradients of sum_r g_r W_r (host-provided upstream gradient g, device array of R):
 // positions, displacements, charges, sigmas, epsilons (user order, n_in each; x3 for
 // vectors) and the 5 softplus parameters per replica (R x 5).  Outputs nullable.
