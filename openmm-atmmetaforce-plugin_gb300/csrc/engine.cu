@@ -1201,6 +1201,8 @@ void Engine::alloc_device() {
     } else {
         a.conv_ctas = 0;
     }
+    a.ends = dalloc<double>(d_allocs_, 2 * (size_t)R_);
+    a.merge_w = dalloc<double>(d_allocs_, (size_t)R_);
     a.results = dalloc<double>(d_allocs_, (size_t)R_ * NUM_RES);
     a.matrix = dalloc<double>(d_allocs_, (size_t)R_ * R_);
     a.beta = reinterpret_cast<double*>(d_params_ + 40);

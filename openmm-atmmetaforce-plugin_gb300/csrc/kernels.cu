@@ -1077,28 +1077,39 @@ __device__ double softcore(double u, double umax, double acore, double ub, doubl
     return (umax - ub) * (zetap - 1.0) * rz + ub;
 }
 
-// The merge of ReferenceATMMetaForceKernels.cpp:82-98 plus the closed-form
-// parameter derivatives of W.
+// What the merge of ReferenceATMMetaForceKernels.cpp:82-98 computes first: u, the
+// soft-core energy and derivative, and the weight sp of the force merge.
+struct MergeHead {
+    double u, usc, fp, x, iee, bfp, sp;
+};
+
+__device__ __forceinline__ MergeHead merge_head(double E1, double E2, const double* p) {
+    MergeHead m;
+    m.u = p[8] > 0 ? E2 - E1 : E1 - E2;
+    m.usc = softcore(m.u, p[5], p[7], p[6], m.fp);
+    m.x = exp(-p[2] * (m.usc - p[3]));
+    m.iee = 1.0 / (1.0 + m.x);
+    m.bfp = (p[1] - p[0]) * m.iee + p[0];
+    m.sp = m.bfp * m.fp;
+    return m;
+}
+
+// The whole merge, with the closed-form parameter derivatives of W.
 __device__ void atm_merge(double E1, double E2, const double* p, double* out) {
     double l1 = p[0], l2 = p[1], alpha = p[2], u0 = p[3], w0 = p[4];
-    double umax = p[5], ub = p[6], acore = p[7], dir = p[8];
-    double u = dir > 0 ? E2 - E1 : E1 - E2;
-    double e0 = dir > 0 ? E1 : E2;
-    double fp;
-    double usc = softcore(u, umax, acore, ub, fp);
-    double x = exp(-alpha * (usc - u0));
-    double ee = 1.0 + x;
-    const double iee = 1.0 / ee, ia = alpha > 0 ? 1.0 / alpha : 0.0;
+    double e0 = p[8] > 0 ? E1 : E2;
+    const MergeHead m = merge_head(E1, E2, p);
+    const double usc = m.usc, x = m.x, iee = m.iee, fp = m.fp, bfp = m.bfp;
+    const double ia = alpha > 0 ? 1.0 / alpha : 0.0;
     double W = 0.0;
-    double L = log(ee);
+    double L = log(1.0 + x);
     if (alpha > 0) W = ((l2 - l1) * ia) * L;
     W += l2 * usc + w0;
-    double bfp = (l2 - l1) * iee + l1;
     out[RES_ENERGY] = e0 + W;
     out[RES_PERT] = usc;
-    out[RES_SP] = bfp * fp;
+    out[RES_SP] = m.sp;
     out[RES_W] = W;
-    out[RES_U] = u;
+    out[RES_U] = m.u;
     out[RES_E0] = e0;
     out[RES_BFP] = bfp;
     out[RES_FP] = fp;
@@ -1121,10 +1132,10 @@ __device__ void atm_merge(double E1, double E2, const double* p, double* out) {
     out[RES_DWDU] = (alpha > 0 ? bfp : l2) * fp;
 }
 
-// Energies of a replica and the ATM merge, one kernel: CTA c of replica r sums
-// the tile energies of the replica's rows c, c + C, ... (C = fin_ctas; rows of
-// state 1, then rows of state 2 or of the difference tiles), warp per row, lanes
-// over its slots, each lane in compensated FP32 (TwoSum: relative error of order
+// End-state energies of a replica and the weight of its force merge, one kernel: CTA c
+// of replica r sums the tile energies of the replica's rows c, c + C, ... (C = fin_ctas;
+// rows of state 1, then rows of state 2 or of the difference tiles), warp per row,
+// lanes over its slots, each lane in compensated FP32 (TwoSum: relative error of order
 // 2^-48 of the summed magnitudes, on the FP32 pipe), the lanes' compensated pairs
 // combined over a shuffle tree and converted to FP64 once per warp, then FP64
 // across warps and CTAs, in a fixed order (no fixed-point range would do:
@@ -1132,7 +1143,16 @@ __device__ void atm_merge(double E1, double E2, const double* p, double* out) {
 // kJ/mol and more, which the soft-core exists to absorb), and writes its two
 // partials; the last CTA of the replica to finish (a counter it resets for the
 // next evaluation) adds the partials in order, the exceptions' and the
-// reciprocal sum's partials, and runs the FP64 merge.
+// reciprocal sum's partials, and runs the head of the FP64 merge.
+//
+// The evaluation waits on this kernel's chain of latencies, not on its work: so a
+// warp's row counts are one load and its rows' energies kFinRows loads in flight, every
+// CTA loads the exceptions' and reciprocal partials before its rows (one warp per
+// quantity: an FP64 add occupies the pipe for 16 cycles per warp), and the rest of the
+// merge (log, derivatives) is left to the output kernel, beside the forces.
+// One 23,558-atom replica 18.5 -> 13.0 us, 22 of them 22 -> 16 us (with the whole merge,
+// the partials after the rows and one row at a time before); the output kernel pays
+// 1 us of it back.
 constexpr int kFinThreads = 256;
 
 // Knuth's TwoSum: s + c carries the running sum exactly up to c's own rounding.
@@ -1154,29 +1174,59 @@ __device__ __forceinline__ void fin_pair_add(float& h, float& l, float hb, float
     l = t - (h - s);
 }
 
+constexpr int kFinRows = 4;  // rows whose energies are in flight at once per warp
+
 __global__ void __launch_bounds__(kFinThreads) k_finalize(Args a) {
     __shared__ double sh_r[2][kFinThreads / 32];
-    __shared__ double sh[5][kFinThreads / 32];
+    __shared__ double sh[5];
     __shared__ int s_last;
     const int C = a.fin_ctas;
     const int r = blockIdx.x / C, c = blockIdx.x - r * C;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const RepDev& R = a.reps[r];
     const int n1 = R.row1_e - R.row1_b, n2 = R.row2_e - R.row2_b;
+    // partials of the exceptions (quantities 0-2, warps 0-2) and of the reciprocal sum
+    // (3, 4): only the last CTA needs them
+    double part = 0.0;
+    if (w < 3)
+        for (int q = R.exc_cta_b + lane; q < R.exc_cta_e; q += 32) part += a.e_part_exc[3 * q + w];
+    else if (w < 5)
+        for (int q = R.conv_cta_b + lane; q < R.conv_cta_e; q += 32) part += a.e_part_conv[2 * q + w - 3];
     float h1 = 0.f, l1 = 0.f, h2 = 0.f, l2 = 0.f;  // compensated sums of the two row kinds
-    for (int k = c + C * w; k < n1 + n2; k += C * (kFinThreads / 32)) {
-        const int row = k < n1 ? R.row1_b + k : R.row2_b + (k - n1);
-        const int n = a.row_count[row];
-        const float2* e = a.e_tile + (size_t)row * a.row_cap;
-        const bool first = k < n1;
-        for (int q = lane; q < n; q += 32) {
-            const float2 v = e[q];
-            if (first) {
-                fin_two_sum(h1, l1, v.x);
-                l1 += v.y;
-            } else {
-                fin_two_sum(h2, l2, v.x);
-                l2 += v.y;
+    const int step = C * (kFinThreads / 32);
+    for (int k0 = c + C * w; k0 < n1 + n2; k0 += 32 * step) {
+        // lane i: the warp's i-th row and its tile count
+        const int km = k0 + lane * step;
+        const int mrow = km < n1 ? R.row1_b + km : R.row2_b + (km - n1);
+        const int mn = km < n1 + n2 ? a.row_count[mrow] : 0;
+        const int rows = min(32, (n1 + n2 - k0 + step - 1) / step);
+        for (int i0 = 0; i0 < rows; i0 += kFinRows) {
+            float2 v[kFinRows];
+#pragma unroll
+            for (int t = 0; t < kFinRows; t++) {
+                const int n = __shfl_sync(FULL_MASK, mn, (i0 + t) & 31), row = __shfl_sync(FULL_MASK, mrow, (i0 + t) & 31);
+                v[t] = i0 + t < rows && lane < n ? a.e_tile[(size_t)row * a.row_cap + lane] : make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int t = 0; t < kFinRows; t++) {
+                if (i0 + t >= rows) break;
+                const int n = __shfl_sync(FULL_MASK, mn, i0 + t), row = __shfl_sync(FULL_MASK, mrow, i0 + t);
+                const bool first = k0 + (i0 + t) * step < n1;
+                float h = first ? h1 : h2, l = first ? l1 : l2;
+                fin_two_sum(h, l, v[t].x);
+                l += v[t].y;
+                for (int q = lane + 32; q < n; q += 32) {
+                    const float2 x = a.e_tile[(size_t)row * a.row_cap + q];
+                    fin_two_sum(h, l, x.x);
+                    l += x.y;
+                }
+                if (first) {
+                    h1 = h;
+                    l1 = l;
+                } else {
+                    h2 = h;
+                    l2 = l;
+                }
             }
         }
     }
@@ -1207,51 +1257,29 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(Args a) {
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // the replica's last CTA: partials of the rows (fixed order), the exceptions
-    // (3) and the reciprocal sum (2)
-    double v[5] = {0, 0, 0, 0, 0};
-    for (int q = R.exc_cta_b + threadIdx.x; q < R.exc_cta_e; q += blockDim.x) {
-        v[0] += a.e_part_exc[3 * q];
-        v[1] += a.e_part_exc[3 * q + 1];
-        v[2] += a.e_part_exc[3 * q + 2];
-    }
-    for (int q = R.conv_cta_b + threadIdx.x; q < R.conv_cta_e; q += blockDim.x) {
-        v[3] += a.e_part_conv[2 * q];
-        v[4] += a.e_part_conv[2 * q + 1];
-    }
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(FULL_MASK, v[k], o);
-        if (lane == 0) sh[k][w] = v[k];
-    }
-    __syncthreads();
-    if (w != 0) return;
-    // warp 0: the CTAs' partials (lane q holds CTAs q, q + 32, ...) and the warps'
-    // sums, each added over a fixed shuffle tree
+    // the replica's last CTA: warps 0-4 their quantity, warp 5 the CTAs' partials of
+    // the rows (lane q holds CTAs q, q + 32, ...), each over a fixed shuffle tree
     double dir1 = 0.0, dir2 = 0.0;
-    {
-        const volatile double* part = a.fin_part + 2 * (size_t)r * C;
+    if (w < 5) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(FULL_MASK, part, o);
+        if (lane == 0) sh[w] = part;
+    } else if (w == 5) {
+        const volatile double* fp = a.fin_part + 2 * (size_t)r * C;
         for (int q = lane; q < C; q += 32) {
-            dir1 += part[2 * q];
-            dir2 += part[2 * q + 1];
+            dir1 += fp[2 * q];
+            dir2 += fp[2 * q + 1];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            dir1 += __shfl_xor_sync(FULL_MASK, dir1, o);
+            dir2 += __shfl_xor_sync(FULL_MASK, dir2, o);
         }
     }
-    double t[5];
-#pragma unroll
-    for (int k = 0; k < 5; k++) t[k] = lane < kFinThreads / 32 ? sh[k][lane] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        dir1 += __shfl_xor_sync(FULL_MASK, dir1, o);
-        dir2 += __shfl_xor_sync(FULL_MASK, dir2, o);
-    }
-#pragma unroll
-    for (int o = (kFinThreads / 32) / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < 5; k++) t[k] += __shfl_xor_sync(FULL_MASK, t[k], o);
-    if (lane == 0) {
+    __syncthreads();
+    if (w == 5 && lane == 0) {
         a.fin_count[r] = 0;  // ready for the next evaluation
-        const double x1 = t[0], x2 = t[1], xd = t[2], c1 = t[3], c2 = t[4];
+        const double x1 = sh[0], x2 = sh[1], xd = sh[2], c1 = sh[3], c2 = sh[4];
         double E1 = dir1 + x1 + c1 + R.e_self + R.e_disp;
         double E2;
         if (a.full) {
@@ -1260,16 +1288,11 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(Args a) {
         } else {
             E2 = E1 + (dir2 + xd + c2);
         }
-        double* out = a.results + (size_t)r * NUM_RES;
+        a.ends[2 * r] = E1;  // the NonbondedForce energy at x and at x + d
+        a.ends[2 * r + 1] = E2;
         // a NonbondedForce outside the variable groups contributes nothing to U_var
-        atm_merge(R.var_nb ? E1 : 0.0, R.var_nb ? E2 : 0.0, R.params, out);
-        out[RES_E1] = E1;  // the NonbondedForce energy at x and at x + d
-        out[RES_E2] = E2;
-        out[RES_STATUS] = (double)a.status->overflow;
-        if (a.io[2])
-            for (int k = 0; k < NUM_RES; k++) a.io[2][(size_t)r * NUM_RES + k] = out[k];
-        if (a.h_results)
-            for (int k = 0; k < NUM_RES; k++) a.h_results[(size_t)r * NUM_RES + k] = out[k];
+        const MergeHead m = merge_head(R.var_nb ? E1 : 0.0, R.var_nb ? E2 : 0.0, R.params);
+        a.merge_w[r] = R.params[8] > 0 ? m.sp : 1.0 - m.sp;
         a.rep_hmax[r] = 0u;  // ready for the next evaluation (the finder has read it)
     }
 }
@@ -1285,20 +1308,48 @@ void launch_finalize(const Args& a, cudaStream_t s) {
 // without a separate copy.
 constexpr int kOutThreads = 256;
 
-// replicas x states energy matrix: beta * (e0(r; dir_s) + W_s(usc_s(u(r; dir_s)))), entry idx
+// Entry idx of the replicas x states energy matrix, beta * (e0(r; dir_s) + W_s(usc_s(u(r;
+// dir_s)))), and on its diagonal the result record of replica r.
 __device__ __forceinline__ void matrix_entry(const Args& a, int idx) {
-    int r = idx / a.R, s = idx % a.R;
-    const double* res = a.results + (size_t)r * NUM_RES;
+    const int r = idx / a.R, s = idx % a.R;
+    const double E1 = a.ends[2 * r], E2 = a.ends[2 * r + 1];
     double out[NUM_RES];
-    bool v = a.reps[r].var_nb;
-    atm_merge(v ? res[RES_E1] : 0.0, v ? res[RES_E2] : 0.0, a.reps[s].params, out);
+    const bool v = a.reps[r].var_nb;
+    atm_merge(v ? E1 : 0.0, v ? E2 : 0.0, a.reps[s].params, out);
     const double e = *a.beta * out[RES_ENERGY];
     a.matrix[idx] = e;
     if (a.h_matrix) a.h_matrix[idx] = e;
+    if (r != s) return;
+    out[RES_E1] = E1;
+    out[RES_E2] = E2;
+    out[RES_STATUS] = (double)a.status->overflow;
+    double* const to[3] = {a.results, a.io[2], a.h_results};
+#pragma unroll
+    for (int t = 0; t < 3; t++)
+        if (to[t])
+            for (int k = 0; k < NUM_RES; k++) to[t][(size_t)r * NUM_RES + k] = out[k];
 }
 
-// The first nmat CTAs compute the matrix (a chain of FP64 functions about as long as
-// the whole force output, so beside it) and hand the status to the host.
+// A warp's nv <= 32 forces to dst: 16-byte words through shared memory where dst allows.
+__device__ __forceinline__ void store_forces(double* dst, const double* f, double* stage, int lane, int nv) {
+    if (nv == 32 && (reinterpret_cast<size_t>(dst) & 15) == 0) {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; k++) stage[3 * lane + k] = f[k];
+        __syncwarp();
+        const double2* src = reinterpret_cast<const double2*>(stage);
+        double2* d2 = reinterpret_cast<double2*>(dst);
+        d2[lane] = src[lane];
+        if (lane < 16) d2[32 + lane] = src[32 + lane];
+    } else if (lane < nv) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) dst[3 * lane + k] = f[k];
+    }
+}
+
+// The first nmat CTAs compute the matrix and the result records (a chain of FP64
+// functions about as long as the whole force output, so beside it) and hand the status
+// to the host.
 __global__ void __launch_bounds__(kOutThreads) k_output(Args a, int nmat) {
     __shared__ double s_f[kOutThreads / 32][96];
     if ((int)blockIdx.x < nmat) {
@@ -1310,14 +1361,12 @@ __global__ void __launch_bounds__(kOutThreads) k_output(Args a, int nmat) {
     const int g = (blockIdx.x - nmat) * kOutThreads + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double* const fo = a.io[1] ? a.io[1] : a.f_out;
     double* const fnb = a.io[3];
-    double f[3] = {0.0, 0.0, 0.0};
+    double f[3] = {0.0, 0.0, 0.0}, fb[3] = {0.0, 0.0, 0.0};
     if (g < a.n_in) {
         const int s = a.slot_of[g];
         const int rep = a.block_rep[s >> 5];
         const RepDev& R = a.reps[rep];
-        const double* res = a.results + (size_t)rep * NUM_RES;
-        const double sp = res[RES_SP];
-        const double wgt = R.params[8] > 0 ? sp : 1.0 - sp;
+        const double wgt = a.merge_w[rep];
         // F1 + w (F2 - F1) in the fixed point of the force sums, w in units of 2^-32
         // (w in [0, 1]: at most 2^32; its rounding is 2^-33 relative to F2 - F1),
         // the product by a 128-bit multiply (floor), then one conversion per
@@ -1332,25 +1381,14 @@ __global__ void __launch_bounds__(kOutThreads) k_output(Args a, int nmat) {
             const unsigned long long lo = (unsigned long long)d * (unsigned long long)w32;
             const long long v = f1 + (long long)(((unsigned long long)hi << 32) | (lo >> 32));
             f[k] = R.var_nb ? fix_scaled(v) : 0.0;
-            if (fnb) fnb[3 * (size_t)g + k] = fix_scaled(f1);
+            if (fnb) fb[k] = fix_scaled(f1);
         }
     }
     const int g0 = g - lane;  // the warp's first atom
     const int nv = min(32, a.n_in - g0);
     if (nv <= 0) return;
-    double* const dst = fo + 3 * (size_t)g0;
-    if (nv == 32 && (reinterpret_cast<size_t>(dst) & 15) == 0) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) s_f[w][3 * lane + k] = f[k];
-        __syncwarp();
-        const double2* src = reinterpret_cast<const double2*>(s_f[w]);
-        double2* d2 = reinterpret_cast<double2*>(dst);
-        d2[lane] = src[lane];
-        if (lane < 16) d2[32 + lane] = src[32 + lane];
-    } else if (lane < nv) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) dst[3 * lane + k] = f[k];
-    }
+    store_forces(fo + 3 * (size_t)g0, f, s_f[w], lane, nv);
+    if (fnb) store_forces(fnb + 3 * (size_t)g0, fb, s_f[w], lane, nv);
 }
 
 void launch_output(const Args& a, cudaStream_t s) {

@@ -317,6 +317,8 @@ struct Args {
     float* influence;         // influence function per replica, [ky][x][kz] at cplx_off / 2
     long long n_real_total;
     // results
+    double* ends;             // R x 2: E1, E2
+    double* merge_w;          // R: the weight of F2 - F1 in the merged force
     double* results;          // R * NUM_RES
     double* matrix;           // R * R
     const double* beta;       // device scalar
