@@ -39,6 +39,8 @@ struct KernelTime {
     double ms;
 };
 
+struct RepLayout;  // one replica's part of the layout (engine.cu)
+
 class Engine {
 public:
     // adjoint: also accumulate the derivatives needed by backward() (difference mode only)
@@ -141,6 +143,7 @@ public:
 
 private:
     void build_layout();
+    void layout_replica(int r, RepLayout& L) const;
     void set_box_constants(RepDev& rd, const ReplicaSpec& s) const;
     static void recip_box(const ReplicaSpec& s, double* r);
     static double min_face_distance(const ReplicaSpec& s);
@@ -155,6 +158,7 @@ private:
     void upload_static();
     void fill_args();
     void update_rep_table();
+    double dispersion_energy(int r);
     void record(cudaStream_t main, const Args& a);
     void pme_transforms(cudaStream_t st, const std::function<void(const char*)>& mark = nullptr);
     // The device mirror of the parameter block, brought up to date on the stream.
@@ -170,6 +174,8 @@ private:
     bool full_ = false;
     bool adjoint_ = false;
     std::vector<ReplicaSpec> specs_;
+    std::vector<double> disp_coef_;  // dispersion coefficient of each replica, where disp_known_
+    std::vector<char> disp_known_;
     std::vector<int> in_off_;
     int n_in_ = 0;
     int NA_ = 0, NB_ = 0, nrows_ = 0;
@@ -205,7 +211,6 @@ private:
     std::vector<int4> row_desc_;
     std::vector<int> ex_start_, dx_start_;
     std::vector<int2> ex_ent_, dx_ent_;
-    std::vector<uint32_t> masks_;             // 32 x 32 exclusion masks (layout build)
     std::vector<uint32_t> masks16_;           // 16 x 16 sub-tile masks (device)
     std::vector<int> exs_start_, dxs_start_;  // per block: its exclusion sub-tiles
     std::vector<int4> exs_ent_, dxs_ent_;     //   (I16, J16, mask16 id, 0)

@@ -86,3 +86,28 @@ def test_noalloc_skips_no_pair(n, edge):
     assert abs(e.item() - E) <= 2e-6 * (sum(abs(v) for v in T.values()) + 1.0)
     # (no pair at all in the sparsest box: both are zero)
     assert np.sqrt(((f.cpu().numpy() - F) ** 2).sum()) <= F_TOL * np.sqrt((F ** 2).sum())
+
+
+@pytest.mark.parametrize("method", [S.PME, S.CUTOFF_PERIODIC], ids=["pme", "rf"])
+def test_dispersion_correction_follows_parameters_and_box(method):
+    """The dispersion correction of each replica after new epsilons of one of them and
+    after a new box, against the oracle."""
+    cases = [S.water_ligand_box(1100, 2.25, [9], [(1.1, 1.0, 1.2)], method, 0.9, seed=80 + k, use_disp_corr=True)
+             for k in range(2)]
+    b = atm.ReplicaBatch([atm.system_from_case(c)[0] for c in cases], 0)
+    pos = np.concatenate([c.pos for c in cases])
+
+    def check(E):
+        for k, c in enumerate(cases):
+            ref = O.atm_eval(c.spec, c.pos, c.displ, c.params)
+            _, _, T = O.nonbonded(c.spec, c.pos)
+            assert abs(E[k] - ref["energy"]) <= 2e-6 * (sum(abs(v) for v in T.values()) + 1.0) + U_TOL
+
+    check(b.evaluate(pos)[0])
+    cases[1].spec.epsilon = cases[1].spec.epsilon * 1.7
+    b.setNonbondedParameters(1, cases[1].spec.charge, cases[1].spec.sigma, cases[1].spec.epsilon)
+    check(b.evaluate(pos)[0])
+    cases[0].spec.box = cases[0].spec.box * 1.01
+    L = cases[0].spec.box
+    b.setPeriodicBoxVectors(0, (L[0], 0, 0), (0, L[1], 0), (0, 0, L[2]))
+    check(b.evaluate(pos)[0])
