@@ -110,6 +110,7 @@ _SIGS = {
     "atm_md_get_list_info": [_vp, _dp, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong), _ip],
     "atm_batch_set_displacements": [_vp, C.c_int, _dp],
     "atm_batch_set_nonbonded_parameters": [_vp, C.c_int, _dp, _dp, _dp],
+    "atm_batch_set_inputs_device": [_vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "atm_batch_backward_device": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "atm_batch_backward": [_vp, _dp, _dp, _dp, _dp, _dp, _dp, _dp],
     "atm_batch_set_profiling": [_vp, C.c_int],

@@ -510,6 +510,13 @@ class ReplicaBatch:
             raise ATMError(1, "wrong number of particle parameters")
         call("atm_batch_set_nonbonded_parameters", self._h, int(replica), _ptr(q), _ptr(s), _ptr(e))
 
+    def setInputsDevice(self, d_displ, d_charge, d_sigma, d_epsilon, d_params, stream=0):
+        """Displacements, charges, sigmas, epsilons and the (R, 5) softplus parameters of
+        every replica from device pointers (ints) of float64 buffers; what equals the
+        batch's is kept.  Waits for the stream."""
+        call("atm_batch_set_inputs_device", self._h, *(C.c_void_p(p) for p in (d_displ, d_charge, d_sigma, d_epsilon,
+                                                                                d_params)), C.c_void_p(stream or None))
+
     def backward(self, g=None):
         """Gradients of sum_r g[r] W_r (g defaults to ones) from the last
         evaluation: dict of positions, displacements (sum n, 3), charge, sigma,

@@ -25,31 +25,48 @@ RES_W = 3
 PARAM_NAMES5 = ("ATMLambda1", "ATMLambda2", "ATMAlpha", "ATMU0", "ATMW0")
 
 
+def _set_inputs_host(batch, cache, displacements, params, charge, sigma, epsilon):
+    """The inputs through host arrays, for tensors of another type, device or shape than the
+    batch's: what differs from the last call's values is set."""
+    R, offs = batch.R, batch.offsets
+    d_np = displacements.detach().cpu().numpy()
+    p_np = params.detach().cpu().numpy()
+    q_np = charge.detach().cpu().numpy()
+    s_np = sigma.detach().cpu().numpy()
+    e_np = epsilon.detach().cpu().numpy()
+    for r in range(R):
+        a, b = offs[r], offs[r + 1]
+        key_d = d_np[a:b].tobytes()
+        if cache.get(("d", r)) != key_d:
+            batch.setDisplacements(r, d_np[a:b])
+            cache[("d", r)] = key_d
+        key_p = q_np[a:b].tobytes() + s_np[a:b].tobytes() + e_np[a:b].tobytes()
+        if cache.get(("p", r)) != key_p:
+            batch.setNonbondedParameters(r, q_np[a:b], s_np[a:b], e_np[a:b])
+            cache[("p", r)] = key_p
+        for k, name in enumerate(PARAM_NAMES5):
+            batch.setParameter(r, name, float(p_np[r, k]))
+
+
 class _ATMSoftplusEnergy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, positions, displacements, params, charge, sigma, epsilon, batch, cache):
-        R, offs = batch.R, batch.offsets
-        d_np = displacements.detach().cpu().numpy()
-        p_np = params.detach().cpu().numpy()
-        q_np = charge.detach().cpu().numpy()
-        s_np = sigma.detach().cpu().numpy()
-        e_np = epsilon.detach().cpu().numpy()
-        for r in range(R):
-            a, b = offs[r], offs[r + 1]
-            key_d = d_np[a:b].tobytes()
-            if cache.get(("d", r)) != key_d:
-                batch.setDisplacements(r, d_np[a:b])
-                cache[("d", r)] = key_d
-            key_p = q_np[a:b].tobytes() + s_np[a:b].tobytes() + e_np[a:b].tobytes()
-            if cache.get(("p", r)) != key_p:
-                batch.setNonbondedParameters(r, q_np[a:b], s_np[a:b], e_np[a:b])
-                cache[("p", r)] = key_p
-            for k, name in enumerate(PARAM_NAMES5):
-                batch.setParameter(r, name, float(p_np[r, k]))
+        R, N = batch.R, int(batch.offsets[-1])
+        dev = positions.device
+        stream = torch.cuda.current_stream(dev).cuda_stream
         pos = positions.detach().contiguous()
+        inputs = [t.detach() for t in (displacements, charge, sigma, epsilon, params)]
+        shapes = [(N, 3), (N,), (N,), (N,), (R, 5)]
+        if all(t.device == dev and t.dtype == torch.float64 and tuple(t.shape) == s
+               for t, s in zip(inputs, shapes)):
+            # compared with the batch's on the device; only what changed is taken over
+            inputs = [t.contiguous() for t in inputs]
+            batch.setInputsDevice(*(t.data_ptr() for t in inputs), stream)
+            cache.clear()
+        else:
+            _set_inputs_host(batch, cache, displacements, params, charge, sigma, epsilon)
         forces = torch.empty_like(pos)
         results = torch.empty((R, NUM_RES), dtype=torch.float64, device=pos.device)
-        stream = torch.cuda.current_stream(pos.device).cuda_stream
         batch.evaluateDevice(pos.data_ptr(), forces.data_ptr(), results.data_ptr(), stream)
         ctx.batch = batch
         ctx.shapes = (positions.shape, R)

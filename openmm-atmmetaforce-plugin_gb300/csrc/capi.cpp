@@ -799,6 +799,14 @@ int atm_batch_set_nonbonded_parameters(atm_batch_t b, int replica, const double*
     API_END
 }
 
+int atm_batch_set_inputs_device(atm_batch_t b, const double* d_displ, const double* d_charge, const double* d_sigma,
+                                const double* d_epsilon, const double* d_params, void* stream) {
+    API_BEGIN
+    REQUIRE(b && d_displ && d_charge && d_sigma && d_epsilon && d_params, ATM_ERR_INVALID_ARGUMENT, "null argument");
+    b->eng->set_inputs_device(d_displ, d_charge, d_sigma, d_epsilon, d_params, (cudaStream_t)stream);
+    API_END
+}
+
 int atm_batch_backward_device(atm_batch_t b, const double* d_g, double* d_dx, double* d_dd, double* d_dq,
                               double* d_dsig, double* d_deps, double* d_dparams, void* stream) {
     API_BEGIN

@@ -206,6 +206,7 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
         crf_ = 3.0 * er / ((2.0 * er + 1.0) * cutoff_);
     }
 
+    e_self_.assign(R_, 0.0);
     disp_coef_.assign(R_, 0.0);
     disp_known_.assign(R_, 0);
 
@@ -234,6 +235,7 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
     h_ctl_[0] = 1;
     h_ctl_[1] = 0;
     CUDA_CHECK(cudaMallocHost(&h_status_, sizeof(Status)));
+    CUDA_CHECK(cudaMallocHost(&h_inputs_, sizeof(double) * (2 + 5 * (size_t)R_)));
     std::memset(h_pos_, 0, sizeof(double) * 3 * (size_t)n_in_);
     int per = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev_));
@@ -260,6 +262,7 @@ Engine::~Engine() {
     cudaFreeHost(h_params_);
     if (d_counts_) cudaFree(d_counts_);
     cudaFreeHost(h_status_);
+    cudaFreeHost(h_inputs_);
     if (ev_fork_) cudaEventDestroy(ev_fork_);
     if (ev_join_) cudaEventDestroy(ev_join_);
     if (s_main_) cudaStreamDestroy(s_main_);
@@ -642,7 +645,13 @@ static void append(std::vector<T>& to, const std::vector<T>& from) {
     to.insert(to.end(), from.begin(), from.end());
 }
 
+// The PME self energy per sum of squared charges.
+double Engine::self_factor() const {
+    return method_ == NonbondedForce::PME ? -kOne4PiEps0 * alpha_ / std::sqrt(kPi) : 0.0;
+}
+
 void Engine::build_layout() {
+    fetch_nonbonded_params();
     orig_.clear();
     slot_of_.assign(n_in_, -1);
     block_rep_.clear();
@@ -739,7 +748,7 @@ void Engine::build_layout() {
         // box and constants
         set_box_constants(rd, s);
         for (int a = 0; a < 3; a++) rd.K[a] = s.grid[a];
-        rd.e_self = (method_ == NonbondedForce::PME) ? -kOne4PiEps0 * alpha_ / std::sqrt(kPi) * L.q2 : 0.0;
+        e_self_[r] = self_factor() * L.q2;
         rd.var_nb = s.var_nb ? 1 : 0;
     }
     exc_cta_first_.push_back((int)exc_ij_.size());
@@ -1122,6 +1131,10 @@ static T* dupload(std::vector<void*>& list, const std::vector<T>& v) {
 
 void Engine::alloc_device() {
     CUDA_CHECK(cudaSetDevice(dev_));
+    if (nb_newer_on_device_) {  // (the same layout in new buffers)
+        fetch_nonbonded_params();
+        refresh_param_tables();
+    }
     destroy_graphs();
     free_device();
     Args& a = A_;
@@ -1162,6 +1175,7 @@ void Engine::alloc_device() {
     a.io = reinterpret_cast<double**>(d_params_ + 8);
     a.orig = dupload(d_allocs_, orig_);
     a.qs = dupload(d_allocs_, qs_);
+    d_nb_ = nullptr;
     a.lj = dupload(d_allocs_, lj_);
     a.displ = dupload(d_allocs_, displ_sorted_);
     a.posq = dalloc<float4>(d_allocs_, NA_);
@@ -1269,6 +1283,7 @@ void Engine::alloc_device() {
     } else {
         a.conv_ctas = 0;
     }
+    a.e_self = dupload(d_allocs_, e_self_);
     a.ends = dalloc<double>(d_allocs_, 2 * (size_t)R_);
     a.merge_w = dalloc<double>(d_allocs_, (size_t)R_);
     a.results = dalloc<double>(d_allocs_, (size_t)R_ * NUM_RES);
@@ -1702,12 +1717,113 @@ void Engine::reorder() { layout_ready_ = false; }
 
 void Engine::set_nonbonded_params(int r, const double* q, const double* sig, const double* eps) {
     if (r < 0 || r >= R_) throw Error(2, "Replica index out of range");
+    fetch_nonbonded_params();
     ReplicaSpec& s = specs_[r];
     std::memcpy(s.q.data(), q, sizeof(double) * (size_t)s.n);
     std::memcpy(s.sig.data(), sig, sizeof(double) * (size_t)s.n);
     std::memcpy(s.eps.data(), eps, sizeof(double) * (size_t)s.n);
     disp_known_[r] = 0;
     layout_ready_ = false;  // scaled charges, LJ pairs, exception charges and self energy follow
+}
+
+void Engine::fetch_nonbonded_params() {
+    if (!nb_newer_on_device_) return;
+    CUDA_CHECK(cudaSetDevice(dev_));
+    CUDA_CHECK(cudaDeviceSynchronize());
+    for (int r = 0; r < R_; r++) {
+        ReplicaSpec& s = specs_[r];
+        std::vector<double>* v[3] = {&s.q, &s.sig, &s.eps};
+        for (int k = 0; k < 3; k++)
+            CUDA_CHECK(cudaMemcpy(v[k]->data(), d_nb_ + k * (size_t)n_in_ + in_off_[r], sizeof(double) * s.n,
+                                  cudaMemcpyDeviceToHost));
+    }
+    nb_newer_on_device_ = false;
+}
+
+void Engine::refresh_param_tables() {
+    const double sqk = std::sqrt(kOne4PiEps0);
+    for (int k = 0; k < NA_; k++) {
+        if (orig_[k] < 0) continue;
+        const ReplicaSpec& s = specs_[block_rep_[k / kTile]];
+        const int i = orig_[k];
+        qs_[k] = (float)(s.q[i] * sqk);
+        lj_[k] = make_float2((float)(0.5 * s.sig[i]), (float)(2.0 * std::sqrt(s.eps[i])));
+    }
+    for (size_t e = 0; e < exc_ij_.size(); e++) {
+        const int4 ij = exc_ij_[e];
+        const ReplicaSpec& s = specs_[ij.z];
+        exc_p_[e].w = kOne4PiEps0 * s.q[ij.x - in_off_[ij.z]] * s.q[ij.y - in_off_[ij.z]];
+    }
+    for (int r = 0; r < R_; r++) {
+        double q2 = 0;
+        for (double q : specs_[r].q) q2 += q * q;
+        e_self_[r] = self_factor() * q2;
+    }
+}
+
+void Engine::set_inputs_device(const double* d_displ, const double* d_q, const double* d_sig, const double* d_eps,
+                               const double* d_params, cudaStream_t stream) {
+    CUDA_CHECK(cudaSetDevice(dev_));
+    int* changed = reinterpret_cast<int*>(h_inputs_);
+    double* h_par = h_inputs_ + 2;
+    changed[0] = changed[1] = changed[2] = layout_ready_ ? 0 : 1;
+    if (layout_ready_) {
+        if (!d_nb_) {
+            d_nb_ = dalloc<double>(d_allocs_, 3 * (size_t)n_in_);
+            for (int r = 0; r < R_; r++) {
+                const ReplicaSpec& s = specs_[r];
+                const std::vector<double>* v[3] = {&s.q, &s.sig, &s.eps};
+                for (int k = 0; k < 3; k++)
+                    CUDA_CHECK(cudaMemcpy(d_nb_ + k * (size_t)n_in_ + in_off_[r], v[k]->data(), sizeof(double) * s.n,
+                                          cudaMemcpyHostToDevice));
+            }
+        }
+        DeviceInputs in{d_displ, d_q, d_sig, d_eps, d_params, d_nb_, d_nb_ + n_in_, d_nb_ + 2 * (size_t)n_in_};
+        CUDA_CHECK(cudaHostGetDevicePointer((void**)&in.changed, changed, 0));
+        CUDA_CHECK(cudaHostGetDevicePointer((void**)&in.h_params, h_par, 0));
+        in.ke = kOne4PiEps0;
+        in.self_factor = self_factor();
+        launch_compare_inputs(A_, in, stream);
+        CUDA_CHECK(cudaGetLastError());
+        CUDA_CHECK(cudaStreamSynchronize(stream));
+        if (!changed[0] && (changed[1] || changed[2])) {
+            launch_update_inputs(A_, in, stream);
+            CUDA_CHECK(cudaGetLastError());
+            // (evaluations asked for on the default stream run on the engine's own)
+            if (!stream) CUDA_CHECK(cudaStreamSynchronize(stream));
+            nb_newer_on_device_ = true;
+            bool disp = false;
+            for (int r = 0; r < R_; r++) {
+                if (changed[2]) disp_known_[r] = 0;
+                disp = disp || (specs_[r].dispersion && periodic_);
+            }
+            if (changed[2] && disp) {
+                fetch_nonbonded_params();  // the dispersion coefficients are summed on the host
+                refresh_param_tables();
+            }
+        }
+    } else {
+        CUDA_CHECK(cudaMemcpyAsync(h_par, d_params, sizeof(double) * 5 * (size_t)R_, cudaMemcpyDeviceToHost, stream));
+        CUDA_CHECK(cudaStreamSynchronize(stream));
+    }
+    if (changed[0]) {
+        // displacements decide the layout: everything through the host
+        std::vector<double> h(6 * (size_t)n_in_);
+        const double* src[4] = {d_displ, d_q, d_sig, d_eps};
+        size_t at[5] = {0, 3, 4, 5, 6};
+        for (int k = 0; k < 4; k++)
+            CUDA_CHECK(cudaMemcpyAsync(h.data() + at[k] * n_in_, src[k], sizeof(double) * (at[k + 1] - at[k]) * n_in_,
+                                       cudaMemcpyDeviceToHost, stream));
+        CUDA_CHECK(cudaStreamSynchronize(stream));
+        for (int r = 0; r < R_; r++) {
+            const size_t o = in_off_[r];
+            set_displacements(r, h.data() + 3 * o);
+            set_nonbonded_params(r, h.data() + 3 * (size_t)n_in_ + o, h.data() + 4 * (size_t)n_in_ + o,
+                                 h.data() + 5 * (size_t)n_in_ + o);
+        }
+    }
+    for (int r = 0; r < R_; r++)
+        for (int k = 0; k < 5; k++) specs_[r].params[k] = h_par[5 * r + k];
 }
 
 void Engine::backward(const double* d_g, double* d_dx, double* d_dd, double* d_dq, double* d_dsig, double* d_deps,

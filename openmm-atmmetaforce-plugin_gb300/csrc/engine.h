@@ -119,6 +119,13 @@ public:
 
     // New charges, sigmas and epsilons of one replica's NonbondedForce (n each).
     void set_nonbonded_params(int r, const double* q, const double* sig, const double* eps);
+    // Displacements, charges, sigmas, epsilons (n_in each, x 3 for vectors) and lambda1,
+    // lambda2, alpha, u0, w0 (R x 5) of every replica from device memory: compared with
+    // the engine's on the device, and only what differs is taken over (new parameters
+    // without the host; new displacements through it, since the layout follows them).
+    // Waits for the stream.
+    void set_inputs_device(const double* d_displ, const double* d_q, const double* d_sig, const double* d_eps,
+                           const double* d_params, cudaStream_t stream);
     bool adjoint() const { return adjoint_; }
     // Gradients of sum_r g[r] W_r from the last evaluation (device pointers on
     // the given stream; outputs nullable, user order).
@@ -159,10 +166,15 @@ private:
     void fill_args();
     void update_rep_table();
     double dispersion_energy(int r);
+    double self_factor() const;
     void record(cudaStream_t main, const Args& a);
     void pme_transforms(cudaStream_t st, const std::function<void(const char*)>& mark = nullptr);
     // The device mirror of the parameter block, brought up to date on the stream.
     void upload_params(cudaStream_t st);
+    // specs_' charges, sigmas and epsilons, and the slot tables made from them, brought up
+    // to date with the device's (after set_inputs_device)
+    void fetch_nonbonded_params();
+    void refresh_param_tables();
     void settle_params();
     // host_results (implied by h_pos_pinned): the result records and the matrix also end
     // in h_results_ / h_matrix_
@@ -176,6 +188,13 @@ private:
     std::vector<ReplicaSpec> specs_;
     std::vector<double> disp_coef_;  // dispersion coefficient of each replica, where disp_known_
     std::vector<char> disp_known_;
+    std::vector<double> e_self_;
+    // the device's charges, sigmas and epsilons (user order, n_in each, one buffer) and
+    // whether they are newer than specs_'
+    double* d_nb_ = nullptr;
+    bool nb_newer_on_device_ = false;
+    // page-locked: 3 change flags (ints), then (from 16 bytes on) the R x 5 softplus parameters
+    double* h_inputs_ = nullptr;
     std::vector<int> in_off_;
     int n_in_ = 0;
     int NA_ = 0, NB_ = 0, nrows_ = 0;

@@ -1280,11 +1280,11 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(Args a) {
     if (w == 5 && lane == 0) {
         a.fin_count[r] = 0;  // ready for the next evaluation
         const double x1 = sh[0], x2 = sh[1], xd = sh[2], c1 = sh[3], c2 = sh[4];
-        double E1 = dir1 + x1 + c1 + R.e_self + R.e_disp;
+        double E1 = dir1 + x1 + c1 + a.e_self[r] + R.e_disp;
         double E2;
         if (a.full) {
             // c2 = E_rec2 - E_rec1, summed directly from the structure-factor update
-            E2 = dir2 + x2 + (c1 + c2) + R.e_self + R.e_disp;
+            E2 = dir2 + x2 + (c1 + c2) + a.e_self[r] + R.e_disp;
         } else {
             E2 = E1 + (dir2 + xd + c2);
         }
@@ -1436,6 +1436,71 @@ void launch_adjoint(const Args& a, const double* g, double* dx, double* dd, doub
                     double* dpar, cudaStream_t s) {
     int n = a.NA > 5 * a.R ? a.NA : 5 * a.R;
     k_adjoint<<<(n + 255) / 256, 256, 0, s>>>(a, g, dx, dd, dq, dsig, deps, dpar);
+}
+
+// One thread per atom: exact comparison with the engine's inputs.  A change is noted
+// in page-locked host memory (any number of threads store the same value).
+__global__ void k_compare_inputs(Args a, DeviceInputs in) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 5 * a.R) in.h_params[i] = in.params[i];
+    if (i >= a.n_in) return;
+    bool d = false;
+    for (int k = 0; k < 3; k++) d = d || in.displ[3 * (size_t)i + k] != a.displ_in[3 * (size_t)i + k];
+    if (d) in.changed[0] = 1;
+    if (in.q[i] != in.cur_q[i]) in.changed[1] = 1;
+    if (in.sig[i] != in.cur_sig[i] || in.eps[i] != in.cur_eps[i]) in.changed[2] = 1;
+}
+
+void launch_compare_inputs(const Args& a, const DeviceInputs& in, cudaStream_t s) {
+    const int n = a.n_in > 5 * a.R ? a.n_in : 5 * a.R;
+    k_compare_inputs<<<(n + 255) / 256, 256, 0, s>>>(a, in);
+}
+
+// New charges, sigmas and epsilons: the slots' scaled values and the exceptions' charge
+// products as the host computes them (FP64, rounded once), and per replica (the last R
+// CTAs) the self energy, summed in a fixed order.
+constexpr int kInThreads = 256;
+
+__global__ void __launch_bounds__(kInThreads) k_update_inputs(Args a, DeviceInputs in, int natom, int nexc) {
+    const int b = blockIdx.x;
+    if (b < natom) {
+        const int i = b * kInThreads + threadIdx.x;
+        if (i >= a.n_in) return;
+        const double q = in.q[i], sig = in.sig[i], eps = in.eps[i];
+        in.cur_q[i] = q;
+        in.cur_sig[i] = sig;
+        in.cur_eps[i] = eps;
+        const int s = a.slot_of[i];
+        a.qs[s] = (float)(q * a.sqrt_ke);
+        a.lj[s] = make_float2((float)(0.5 * sig), (float)(2.0 * sqrt(eps)));
+    } else if (b < natom + nexc) {
+        const int e = (b - natom) * kInThreads + threadIdx.x;
+        if (e >= a.n_exc) return;
+        const int4 ij = a.exc_ij[e];
+        a.exc_p[e].w = in.ke * in.q[ij.x] * in.q[ij.y];
+    } else {
+        __shared__ double red[kInThreads / 32];
+        const RepDev& R = a.reps[b - natom - nexc];
+        double t = 0.0;
+        for (int i = threadIdx.x; i < R.n; i += kInThreads) {
+            const double q = in.q[R.in_off + i];
+            t += q * q;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL_MASK, t, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            t = 0.0;
+            for (int w = 0; w < kInThreads / 32; w++) t += red[w];
+            a.e_self[b - natom - nexc] = in.self_factor * t;
+        }
+    }
+}
+
+void launch_update_inputs(const Args& a, const DeviceInputs& in, cudaStream_t s) {
+    const int natom = (a.n_in + kInThreads - 1) / kInThreads, nexc = (a.n_exc + kInThreads - 1) / kInThreads;
+    k_update_inputs<<<natom + nexc + a.R, kInThreads, 0, s>>>(a, in, natom, nexc);
 }
 
 }  // namespace atm

@@ -107,7 +107,6 @@ struct RepDev {
     int tw_off[3];            // FFT twiddle tables of the three grid dimensions
     int fft_plan[3];          // FFT stage plans per dimension: first stage | stage count << 24
     int pad0[1];
-    double e_self;            // PME self energy (FP64, host)
     double e_disp;            // dispersion correction (FP64, host)
     double params[9];         // ATM globals
     // Triclinic boxes, OpenMM's reduced form: a = (box[0], 0, 0),
@@ -236,8 +235,8 @@ struct Args {
                               // state-1 nonbonded force (3*n_in); null: unused
     // slot arrays
     const int* orig;          // NA: user index within the replica, -1 for padding
-    const float* qs;          // NA: charge * sqrt(1/(4 pi eps0))
-    const float2* lj;         // NA: (sigma/2, 2 sqrt(eps))
+    float* qs;                // NA: charge * sqrt(1/(4 pi eps0))
+    float2* lj;               // NA: (sigma/2, 2 sqrt(eps))
     const float4* displ;      // NA: displacement (sorted)
     float4* posq;             // NA: wrapped positions + scaled charge (state 1)
     float4* posq2;            // NA: state 2 (full mode) or null
@@ -284,7 +283,7 @@ struct Args {
     // exceptions (user-order indices, grouped by replica)
     int n_exc;
     const int4* exc_ij;       // (i_in, j_in, replica, cross)
-    const ExcParam* exc_p;    // (chargeProd*ke, sigma, epsilon, q_i q_j ke)
+    ExcParam* exc_p;          // (chargeProd*ke, sigma, epsilon, q_i q_j ke)
     double* e_part_exc;       // 3 per CTA: state 1, state 2, difference
     int exc_ctas;
     const int* exc_cta_first; // first exception of each CTA
@@ -317,6 +316,7 @@ struct Args {
     float* influence;         // influence function per replica, [ky][x][kz] at cplx_off / 2
     long long n_real_total;
     // results
+    double* e_self;           // R: PME self energies
     double* ends;             // R x 2: E1, E2
     double* merge_w;          // R: the weight of F2 - F1 in the merged force
     double* results;          // R * NUM_RES
@@ -354,6 +354,19 @@ void launch_output(const Args& a, cudaStream_t s);
 // vectors) and the 5 softplus parameters per replica (R x 5).  Outputs nullable.
 void launch_adjoint(const Args& a, const double* g, double* dx, double* dd, double* dq, double* dsig, double* deps,
                     double* dpar, cudaStream_t s);
+// Inputs of a differentiable call that live on the device: which of them differ from
+// what the engine holds (changed, page-locked: displacements, charges, sigmas or
+// epsilons), the R x 5 softplus parameters to the host, and the tables that follow
+// from new charges, sigmas and epsilons.
+struct DeviceInputs {
+    const double *displ, *q, *sig, *eps, *params;  // the caller's
+    double *cur_q, *cur_sig, *cur_eps;             // the engine's copies (user order)
+    int* changed;                                  // host, 3 flags
+    double* h_params;                              // host, R x 5
+    double ke, self_factor;                        // 1/(4 pi eps0); self energy per q^2
+};
+void launch_compare_inputs(const Args& a, const DeviceInputs& in, cudaStream_t s);
+void launch_update_inputs(const Args& a, const DeviceInputs& in, cudaStream_t s);
 int tiles_kernel_blocks_per_sm();
 int find_warps_per_sm();
 constexpr int kTileThreads = 256;
