@@ -1200,6 +1200,10 @@ void Engine::alloc_device() {
     a.bb_h = dalloc<float4>(d_allocs_, NB_);
     a.bb_c2 = full_ ? dalloc<float4>(d_allocs_, NB_) : nullptr;
     a.bb_h2 = full_ ? dalloc<float4>(d_allocs_, NB_) : nullptr;
+    a.hb_c = dalloc<float4>(d_allocs_, 2 * (size_t)NB_);
+    a.hb_h = dalloc<float4>(d_allocs_, 2 * (size_t)NB_);
+    a.hb_c2 = full_ ? dalloc<float4>(d_allocs_, 2 * (size_t)NB_) : nullptr;
+    a.hb_h2 = full_ ? dalloc<float4>(d_allocs_, 2 * (size_t)NB_) : nullptr;
     a.row_desc = dupload(d_allocs_, row_desc_);
     a.row_count = dalloc<int>(d_allocs_, nrows_);
     a.row_tbase = dalloc<int>(d_allocs_, nrows_);

@@ -41,16 +41,28 @@ __device__ __forceinline__ float wrapf(float x, float L, float iL) { return x - 
 // ---------------------------------------------------------------------------
 // prepare: one warp per block
 // ---------------------------------------------------------------------------
-// Bounding box of a block (minimum image relative to its first atom); h.w
-// receives the number of real (non-padding) atoms of the block.
-__device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDev& R, float4* c, float4* h,
-                                          int lane, int nreal) {
+// Bounding box of a block (minimum image relative to its first atom); h.w receives
+// the number of real (non-padding) atoms of the block.  With hc, also the boxes of its
+// two halves, whose h.w receives the largest distance of an atom from the box centre.
+__device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDev& R, int b, float4* c, float4* h,
+                                          float4* hc, float4* hh, int lane, int nreal) {
     float x0 = __shfl_sync(FULL_MASK, x, 0), y0 = __shfl_sync(FULL_MASK, y, 0), z0 = __shfl_sync(FULL_MASK, z, 0);
     float dx = x - x0, dy = y - y0, dz = z - z0;
     min_image3(dx, dy, dz, R);
     float lx = dx, ly = dy, lz = dz, hx = dx, hy = dy, hz = dz;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 1; o <= 16; o <<= 1) {
+        if (o == 16 && hc) {
+            const float cx = 0.5f * (lx + hx), cy = 0.5f * (ly + hy), cz = 0.5f * (lz + hz);
+            float r2 = (dx - cx) * (dx - cx) + (dy - cy) * (dy - cy) + (dz - cz) * (dz - cz);
+#pragma unroll
+            for (int p = 1; p <= 8; p <<= 1) r2 = fmaxf(r2, __shfl_xor_sync(FULL_MASK, r2, p));
+            if ((lane & 15) == 0) {
+                const int q = 2 * b + (lane >> 4);
+                hc[q] = make_float4(x0 + cx, y0 + cy, z0 + cz, 0.f);
+                hh[q] = make_float4(0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz), sqrtf(r2));
+            }
+        }
         lx = fminf(lx, __shfl_xor_sync(FULL_MASK, lx, o));
         ly = fminf(ly, __shfl_xor_sync(FULL_MASK, ly, o));
         lz = fminf(lz, __shfl_xor_sync(FULL_MASK, lz, o));
@@ -59,8 +71,8 @@ __device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDe
         hz = fmaxf(hz, __shfl_xor_sync(FULL_MASK, hz, o));
     }
     if (lane == 0) {
-        *c = make_float4(x0 + 0.5f * (lx + hx), y0 + 0.5f * (ly + hy), z0 + 0.5f * (lz + hz), 0.f);
-        *h = make_float4(0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz), __int_as_float(nreal));
+        c[b] = make_float4(x0 + 0.5f * (lx + hx), y0 + 0.5f * (ly + hy), z0 + 0.5f * (lz + hz), 0.f);
+        h[b] = make_float4(0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz), __int_as_float(nreal));
     }
 }
 
@@ -140,7 +152,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
         for (int k = 0; k < 6; k++) a.F[(size_t)k * a.NA + s] = 0ull;
         if (a.adjoint)
             for (int k = 0; k < 3; k++) a.D[(size_t)k * a.NA + s] = 0ull;
-        warp_bbox(x, y, z, R, &a.bb_c[b], &a.bb_h[b], lane, nreal);
+        warp_bbox(x, y, z, R, b, a.bb_c, a.bb_h, a.any_tric ? a.hb_c : nullptr, a.hb_h, lane, nreal);
         if (R.tric && lane == 0) {  // (lane 0 wrote the box)
             const float4 h = a.bb_h[b];
             atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));
@@ -150,7 +162,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
             float x2 = x + d.x, y2 = y + d.y, z2 = z + d.z;
             wrap3(x2, y2, z2, R);
             a.posq2[s] = make_float4(x2, y2, z2, q);
-            warp_bbox(x2, y2, z2, R, &a.bb_c2[b], &a.bb_h2[b], lane, nreal);
+            warp_bbox(x2, y2, z2, R, b, a.bb_c2, a.bb_h2, a.any_tric ? a.hb_c2 : nullptr, a.hb_h2, lane,
+                      nreal);
             if (R.tric && lane == 0) {
                 const float4 h = a.bb_h2[b];
                 atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));

@@ -250,6 +250,8 @@ struct Args {
     float4* bb_h;             // NB: half extents
     float4* bb_c2;            // NB: state 2 (full mode)
     float4* bb_h2;
+    float4 *hb_c, *hb_h;      // 2 NB: the same of the half blocks (triclinic batches; h.w: radius
+    float4 *hb_c2, *hb_h2;    //   about the centre)
     // rows and tiles
     const int4* row_desc;     // nrows: (I, kind, replica, part | parts << 8)
     int* row_count;           // nrows

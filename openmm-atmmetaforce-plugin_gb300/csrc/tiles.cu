@@ -445,6 +445,84 @@ __device__ __forceinline__ int row_atoms(const Args& a, const RepDev& R, int I, 
     return natom;
 }
 
+// Triclinic rows that need per-pair images list every atom of a candidate block, so
+// their tiles' groups of 16 j slots are half blocks (but for those after a partial
+// block).  Which of them can hold a pair within the cutoff of each half of block I: by
+// the half blocks' boxes and spheres, at the image of their centres, which is that of
+// any such pair when cutoff plus both half extents stay below half the box along
+// every axis (the reduced box's images tile space by such boxes).  A group left out
+// holds only terms that are exactly zero: the sums are the same bits.  list: the groups
+// kept for half 0, from list[kMaxGroups] on those for half 1; returns their numbers.
+// 4 x 8,009 atoms in a rhombic dodecahedral cell: k_tiles 210 -> 151 us, k_find 34 -> 46
+// (every listed atom against the half's box instead: 127 and 74).
+constexpr int kMaxGroups = kStageAtoms / kHalf;
+static_assert(kMaxGroups <= 256 && 2 * kMaxGroups <= 32 * (int)sizeof(float4), "the lists take the i positions' place");
+
+__device__ __noinline__ int2 keep_groups(const Args& a, const RepDev& R, int I, int kind, int lane, const int* stage,
+                                         int natom, unsigned char* list) {
+    const ImgBox B = img_box(R);
+    const float4* C = kind == ROW_STATE2 ? a.hb_c2 : a.hb_c;
+    const float4* H = kind == ROW_STATE2 ? a.hb_h2 : a.hb_h;
+    const bool g2 = kind == ROW_DIFF2;
+    const float rc = sqrtf(a.rcl2) * 1.0001f;
+    float4 ci[2] = {C[2 * I], C[2 * I + 1]}, hi[2] = {H[2 * I], H[2 * I + 1]};
+    const float4 di = a.block_d[I];
+    const int ng = (natom + kHalf - 1) / kHalf;
+    const unsigned lt = (1u << lane) - 1u;
+    int2 n = make_int2(0, 0);
+    for (int g0 = 0; g0 < ng; g0 += 32) {
+        const int g = g0 + lane;
+        bool near[2] = {g < ng, g < ng};
+        if (g < ng) {
+            const int j0 = stage[kHalf * g], j1 = kHalf * g + kHalf <= natom ? stage[kHalf * g + kHalf - 1] : -1;
+            if ((j0 & (kHalf - 1)) == 0 && j1 == j0 + kHalf - 1) {
+                const float4 cj = C[j0 / kHalf], hj = H[j0 / kHalf];
+                float ox = cj.x, oy = cj.y, oz = cj.z;
+                if (g2) {
+                    const float4 dj = a.block_d[j0 / kTile];
+                    ox += dj.x - di.x;
+                    oy += dj.y - di.y;
+                    oz += dj.z - di.z;
+                }
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const float hx = hi[q].x + hj.x, hy = hi[q].y + hj.y, hz = hi[q].z + hj.z;
+                    float dx = ox - ci[q].x, dy = oy - ci[q].y, dz = oz - ci[q].z;
+                    min_image_b(dx, dy, dz, B);
+                    const float rr = rc + hi[q].w + hj.w;
+                    // (written so that a distance that is no number keeps its group)
+                    const bool far = box_gap2(dx, dy, dz, hx, hy, hz) >= rc * rc || dx * dx + dy * dy + dz * dz >= rr * rr;
+                    near[q] = !far || rc + hx >= 0.499f * B.Lx || rc + hy >= 0.499f * B.Ly || rc + hz >= 0.499f * B.Lz;
+                }
+            }
+        }
+        const unsigned b0 = __ballot_sync(FULL_MASK, near[0]), b1 = __ballot_sync(FULL_MASK, near[1]);
+        if (near[0]) list[n.x + __popc(b0 & lt)] = (unsigned char)g;
+        if (near[1]) list[kMaxGroups + n.y + __popc(b1 & lt)] = (unsigned char)g;
+        n.x += __popc(b0);
+        n.y += __popc(b1);
+    }
+    __syncwarp();
+    return n;
+}
+
+// The tiles of the kept groups: j slots to out (16 per tile, consecutive) and tile
+// entries, half 0's, then half 1's; two tiles per step.
+__device__ __noinline__ void emit_groups(int I, int zword, int lane, const int* stage, int natom,
+                                         const unsigned char* list, int2 n, int* out, int4* tiles, int slot) {
+    const int l = lane & (kHalf - 1);
+#pragma unroll 4
+    for (int k = lane >> 4; k < n.x + n.y; k += 2) {
+        const int half = k >= n.x ? 1 : 0;
+        const int g = list[half ? kMaxGroups + k - n.x : k];
+        const int cnt = min(kHalf, natom - kHalf * g);
+        out[kHalf * k + l] = l < cnt ? stage[kHalf * g + l] : -1;
+        if (l == 0)
+            tiles[k] = make_int4(2 * I + half, 0, zword | (1 << 30),
+                                 (int)((unsigned)cnt | ((unsigned)(slot + k) << 20) | (1u << 31)));
+    }
+}
+
 // The tiles of one row (one warp; stage and ipos: the warp's shared memory).
 template <bool TRIC>
 __device__ __forceinline__ void find_row(const Args& a, int row, int lane, int* stage, float4* ipos) {
@@ -515,7 +593,15 @@ __device__ __forceinline__ void find_row(const Args& a, int row, int lane, int* 
     const int4* se = diff ? a.dxs_ent : a.exs_ent;
     const int s0 = ss[I];
     const int nblock = part == 0 ? ss[I + 1] - s0 : 0;
-    const int nta = (nA + kHalf - 1) / kHalf, ntb = (nB + kHalf - 1) / kHalf;
+    int nta = (nA + kHalf - 1) / kHalf, ntb = (nB + kHalf - 1) / kHalf;
+    // (the group lists take the place of the i positions, which only the exact cut needs)
+    unsigned char* groups = reinterpret_cast<unsigned char*>(ipos);
+    const bool grouped = TRIC && all_images && staged;
+    if (grouped) {
+        const int2 kept = keep_groups(a, R, I, kind, lane, stage, natom, groups);
+        nta = kept.x;
+        ntb = kept.y;
+    }
     int n = nblock + nta + ntb;
     const bool filler = n & 1;
     n += filler ? 1 : 0;
@@ -538,7 +624,10 @@ __device__ __forceinline__ void find_row(const Args& a, int row, int lane, int* 
     }
     int* outA = a.tile_j + (size_t)(tbase + nblock) * kHalf;
     int* outB = outA + (size_t)nta * kHalf;
-    if (flagged) {
+    const int zword = row | (kind << 28);
+    if (grouped) {
+        emit_groups(I, zword, lane, stage, natom, groups, make_int2(nta, ntb), outA, a.tiles + tbase + nblock, nblock);
+    } else if (flagged) {
         int ka = 0, kb = 0;
         for (int g = 0; g < natom; g += 32) {
             const int k = g + lane;
@@ -563,14 +652,15 @@ __device__ __forceinline__ void find_row(const Args& a, int row, int lane, int* 
         row_atoms<false, TRIC>(a, R, I, kind, ci, hi, ee, e0, e1, lane, outB, natom, ipos, raw, part, nparts, false,
                          all_images);
     }
-    for (int k = nA + lane; k < kHalf * nta; k += 32) outA[k] = -1;
-    for (int k = nB + lane; k < kHalf * ntb; k += 32) outB[k] = -1;
-    const int zword = row | (kind << 28);
+    if (!grouped) {
+        for (int k = nA + lane; k < kHalf * nta; k += 32) outA[k] = -1;
+        for (int k = nB + lane; k < kHalf * ntb; k += 32) outB[k] = -1;
+    }
     for (int k = lane; k < nblock; k += 32) {
         const int4 e = se[s0 + k];
         a.tiles[tbase + k] = make_int4(e.x, e.y, zword, (int)((unsigned)(e.z + 1) | ((unsigned)k << 20) | (pbc << 31)));
     }
-    for (int k = lane; k < nta + ntb; k += 32) {
+    for (int k = lane; k < nta + ntb && !grouped; k += 32) {
         const bool hb = k >= nta;
         const int kk = hb ? k - nta : k;
         const int cnt = min(kHalf, (hb ? nB : nA) - kHalf * kk);
@@ -694,21 +784,19 @@ __device__ __forceinline__ void pair_eval(float r2, float qq, float sig, float e
 // a constant offset per unrolled step), j forces travel with their slot by
 // shuffles within the half.  MASKED: a per-lane bit mask of the pairs to
 // count (exclusions, padding); unmasked tiles park their padding j slots far away.
-template <int METHOD, bool PBC, bool DIFF, bool MASKED>
+template <int METHOD, bool DIFF, bool MASKED>
 __device__ __forceinline__ void tile_steps(const float4* __restrict__ sp, const float2* __restrict__ sl, float4 pi,
-                                           float2 li, unsigned mask, int lane, const ImgBox& B, float rc2,
-                                           float alpha, float krf, float crf, float3& fi, float3& fj, float& e32,
-                                           float2& ec) {
+                                           float2 li, unsigned mask, int lane, float rc2, float alpha, float krf,
+                                           float crf, float3& fi, float3& fj, float& e32, float2& ec) {
     const int src = (lane & kHalf) | ((lane + 1) & (kHalf - 1));  // next lane of this half
     // the unmasked atom tiles carry most pairs; the other variants stay compact
     // so that the hot loop keeps the instruction cache
-    constexpr int kUnroll = (!PBC && !DIFF) ? (MASKED ? 4 : 8) : 2;
+    constexpr int kUnroll = !DIFF ? (MASKED ? 4 : 8) : 2;
 #pragma unroll kUnroll
     for (int k = 0; k < kHalf; k++) {
         const float4 pj = sp[k];
         const float2 lj = sl[k];
-        float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-        if (PBC) min_image_b(dx, dy, dz, B);
+        const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
         const float r2 = dx * dx + dy * dy + dz * dz;
         const bool inc = MASKED ? (((mask >> k) & 1u) && r2 < rc2) : r2 < rc2;
         float e, fr;
@@ -730,6 +818,60 @@ __device__ __forceinline__ void tile_steps(const float4* __restrict__ sp, const 
         fj.y = __shfl_sync(FULL_MASK, fmaf(fr, dy, fj.y), src);
         fj.z = __shfl_sync(FULL_MASK, fmaf(fr, dz, fj.z), src);
     }
+}
+
+// The same pairs when every pair needs its own minimum image (small or triclinic
+// boxes, whose rows are not cut atom by atom: most of their pair slots lie beyond the
+// cutoff).  A first loop marks the pairs within it, a second evaluates the steps at
+// which any lane of the warp has one; between two such steps the j sums move by as
+// many slots as were left out.  A pair left out is one whose terms are exactly zero
+// in tile_steps, so the sums are the same bits.  4 x 8,009 atoms in a rhombic
+// dodecahedral cell: k_tiles 237 -> 210 us.
+template <int METHOD, bool DIFF>
+__device__ __forceinline__ void tile_steps_img(const float4* __restrict__ sp, const float2* __restrict__ sl, float4 pi,
+                                               float2 li, unsigned mask, int lane, const ImgBox& B, float rc2,
+                                               float alpha, float krf, float crf, float3& fi, float3& fj, float& e32,
+                                               float2& ec) {
+    unsigned in = 0u;
+#pragma unroll 4
+    for (int k = 0; k < kHalf; k++) {
+        const float4 pj = sp[k];
+        float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+        min_image_b(dx, dy, dz, B);
+        const float r2 = dx * dx + dy * dy + dz * dz;
+        in |= r2 < rc2 ? 1u << k : 0u;
+    }
+    in &= mask;
+    int at = 0;  // lane l of a half holds the j sums of slot (l + at) & 15
+    for (unsigned steps = __reduce_or_sync(FULL_MASK, in); steps; steps &= steps - 1) {
+        const int k = __ffs(steps) - 1;
+        const int src = (lane & kHalf) | ((lane + k - at) & (kHalf - 1));
+        fj.x = __shfl_sync(FULL_MASK, fj.x, src);
+        fj.y = __shfl_sync(FULL_MASK, fj.y, src);
+        fj.z = __shfl_sync(FULL_MASK, fj.z, src);
+        at = k;
+        if ((in >> k) & 1u) {
+            const float4 pj = sp[k];
+            const float2 lj = sl[k];
+            float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+            min_image_b(dx, dy, dz, B);
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            float e, fr;
+            pair_eval<METHOD>(r2, pi.w * pj.w, li.x + lj.x, li.y * lj.y, alpha, krf, crf, e, fr);
+            if (DIFF) two_sum_add(ec.x, ec.y, e);
+            else e32 += e;
+            fi.x = fmaf(-fr, dx, fi.x);
+            fi.y = fmaf(-fr, dy, fi.y);
+            fi.z = fmaf(-fr, dz, fi.z);
+            fj.x = fmaf(fr, dx, fj.x);
+            fj.y = fmaf(fr, dy, fj.y);
+            fj.z = fmaf(fr, dz, fj.z);
+        }
+    }
+    const int src = (lane & kHalf) | ((lane - at) & (kHalf - 1));  // back to the lane's own slot
+    fj.x = __shfl_sync(FULL_MASK, fj.x, src);
+    fj.y = __shfl_sync(FULL_MASK, fj.y, src);
+    fj.z = __shfl_sync(FULL_MASK, fj.z, src);
 }
 
 // Two FP32 values in one 64-bit register pair, for the packed FP32 instructions
@@ -1095,24 +1237,20 @@ __device__ __forceinline__ void tile_pairs(const Args& a, int cur, int cur_end, 
                                               crf, fi, fj, ec, ai, aj);
         } else if (diff) {
             if (pbc_w)
-                tile_steps<METHOD, true, true, true>(spl, sll, pi, li, mask, lane, img_box(R), rc2,
-                                                     alpha, krf, crf, fi, fj, e32, ec);
+                tile_steps_img<METHOD, true>(spl, sll, pi, li, mask, lane, img_box(R), rc2, alpha, krf, crf, fi, fj,
+                                             e32, ec);
             else if (masked)
-                tile_steps<METHOD, false, true, true>(spl, sll, pi, li, mask, lane, img_box(R), rc2,
-                                                      alpha, krf, crf, fi, fj, e32, ec);
+                tile_steps<METHOD, true, true>(spl, sll, pi, li, mask, lane, rc2, alpha, krf, crf, fi, fj, e32, ec);
             else
-                tile_steps<METHOD, false, true, false>(spl, sll, pi, li, mask, lane, img_box(R), rc2,
-                                                       alpha, krf, crf, fi, fj, e32, ec);
+                tile_steps<METHOD, true, false>(spl, sll, pi, li, mask, lane, rc2, alpha, krf, crf, fi, fj, e32, ec);
         } else {
             if (pbc_w)
-                tile_steps<METHOD, true, false, true>(spl, sll, pi, li, mask, lane, img_box(R), rc2,
-                                                      alpha, krf, crf, fi, fj, e32, ec);
+                tile_steps_img<METHOD, false>(spl, sll, pi, li, mask, lane, img_box(R), rc2, alpha, krf, crf, fi, fj,
+                                              e32, ec);
             else if (masked)
-                tile_steps<METHOD, false, false, true>(spl, sll, pi, li, mask, lane, img_box(R), rc2,
-                                                       alpha, krf, crf, fi, fj, e32, ec);
+                tile_steps<METHOD, false, true>(spl, sll, pi, li, mask, lane, rc2, alpha, krf, crf, fi, fj, e32, ec);
             else
-                tile_steps<METHOD, false, false, false>(spl, sll, pi, li, mask, lane, img_box(R), rc2,
-                                                        alpha, krf, crf, fi, fj, e32, ec);
+                tile_steps<METHOD, false, false>(spl, sll, pi, li, mask, lane, rc2, alpha, krf, crf, fi, fj, e32, ec);
         }
         __syncwarp();
         // the lane's bookkeeping, kept in shared memory across the pair loop

@@ -111,3 +111,18 @@ def test_dispersion_correction_follows_parameters_and_box(method):
     L = cases[0].spec.box
     b.setPeriodicBoxVectors(0, (L[0], 0, 0), (0, L[1], 0), (0, 0, L[2]))
     check(b.evaluate(pos)[0])
+
+
+@pytest.mark.parametrize("diff", [0, 1], ids=["two-states", "difference"])
+@pytest.mark.parametrize("n,L,ligand", [(1506, 2.78, 9), (2703, 3.4, 33), (8009, 4.86, 29)])
+def test_triclinic_rows_by_groups(n, L, ligand, diff):
+    """Rhombic dodecahedral cells whose rows keep or drop whole groups of j slots: too
+    small for any group to be dropped, partial blocks before the moving ones (their
+    groups straddle half blocks), and a cell where most groups are dropped."""
+    c = S.triclinic_water_ligand_box(n, (L, L, L * 0.5 ** 0.5), (0.0, 0.5 * L, 0.5 * L), [ligand],
+                                     [(0.35 * L, 0.35 * L, 0.3 * L)], S.PME, 0.9, seed=120 + ligand)
+    b = atm.ReplicaBatch([atm.system_from_case(c)[0]], 0, {"DifferencePath": diff})
+    E, F, r = b.evaluate(c.pos)
+    ref = O.atm_eval(c.spec, c.pos, c.displ, c.params)
+    assert abs(r[0]["pert"] - ref["usc"]) <= U_TOL
+    assert np.sqrt(((F - ref["forces"]) ** 2).sum() / (ref["forces"] ** 2).sum()) <= F_TOL
