@@ -212,7 +212,10 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
 
     CUDA_CHECK(cudaSetDevice(dev_));
     CUDA_CHECK(cudaStreamCreateWithFlags(&s_main_, cudaStreamNonBlocking));
-    CUDA_CHECK(cudaStreamCreateWithFlags(&s_pme_, cudaStreamNonBlocking));
+    // the PME chain's CTAs go first wherever one ends (Engine::tile_launch_grid)
+    int prio_least = 0, prio_greatest = 0;
+    CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest));
+    CUDA_CHECK(cudaStreamCreateWithPriority(&s_pme_, cudaStreamNonBlocking, prio_greatest));
     CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     CUDA_CHECK(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
     CUDA_CHECK(cudaMallocHost(&h_pos_, sizeof(double) * 3 * (size_t)n_in_));
@@ -1338,11 +1341,23 @@ void Engine::update_rep_table() {
 // One evaluation: the kernel sequence (captured once into a CUDA graph)
 // ---------------------------------------------------------------------------
 
-// Hand the pair tiles out from a counter when the warps of the tile kernel get
-// many tiles each (about 15 tiles per row); a few per warp go in a fixed stride.
+// The pair tiles of large batches are handed out from a counter to persistent CTAs (rows
+// before their split into parts at least the resident warps); smaller ones get about one
+// pass per warp (28 tile pairs a row at the benchmarked densities, the rest of a longer
+// list in strides), so that CTAs end all the time and the PME chain's kernels, whose
+// stream has the higher priority, start beside the pair tiles instead of after them:
+// persistent CTAs fill every SM until the list is done.  Persistent / one pass, us:
+// 23,558 atoms, 50 MD steps 7200 / 6630, PME context 285 / 281; 8 x 12,000 (3,016 rows,
+// 4,864 warps), 20 MD steps 7340 / 6750, boxes of three sizes 379 / 372; 22 x 23,558
+// (16,280 rows) 1006 / 1031, 8 x 60,000 1184 / 1230.
 int Engine::tile_dynamic() const {
     const long long warps = (long long)tile_grid_ * (kTileThreads / 32);
-    return (long long)nrows_ * 15 >= 16 * warps ? 1 : 0;
+    return nrows_ / row_parts_ >= warps ? 1 : 0;
+}
+
+int Engine::tile_launch_grid() const {
+    if (A_.tile_dynamic) return tile_grid_;
+    return std::max(tile_grid_, (int)(4.5 * (nrows_ / row_parts_)));
 }
 
 int Engine::launches_per_eval() const {
@@ -1397,7 +1412,7 @@ void Engine::record(cudaStream_t st, const Args& a) {
         launch_find_tiles(a, st);
     } else {
         launch_find(a, st);
-        launch_tiles(a, tile_grid_, st);
+        launch_tiles(a, tile_launch_grid(), st);
     }
     if (!pme) launch_exceptions(a, st);
     if (pme && tune_pme_stream_) CUDA_CHECK(cudaStreamWaitEvent(st, ev_join_, 0));
@@ -1497,7 +1512,7 @@ void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos_pin
             } else {
                 launch_find(a, st);
                 mark("find");
-                launch_tiles(a, tile_grid_, st);
+                launch_tiles(a, tile_launch_grid(), st);
                 mark("tiles");
             }
             launch_exceptions(a, st);
@@ -1533,7 +1548,7 @@ void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos_pin
                     throw;
                 }
                 CUDA_CHECK(cudaStreamEndCapture(s_main_, &g));
-                CUDA_CHECK(cudaGraphInstantiate(&gx, g, 0));
+                CUDA_CHECK(cudaGraphInstantiate(&gx, g, cudaGraphInstantiateFlagUseNodePriority));
                 CUDA_CHECK(cudaGraphDestroy(g));
             }
             CUDA_CHECK(cudaGraphLaunch(gx, st));
