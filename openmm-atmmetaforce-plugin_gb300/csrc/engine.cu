@@ -1203,6 +1203,11 @@ void Engine::alloc_device() {
     a.bb_h = dalloc<float4>(d_allocs_, NB_);
     a.bb_c2 = full_ ? dalloc<float4>(d_allocs_, NB_) : nullptr;
     a.bb_h2 = full_ ? dalloc<float4>(d_allocs_, NB_) : nullptr;
+    const size_t noct = ((size_t)NB_ + 7) / 8;
+    a.oct_c = dalloc<float4>(d_allocs_, noct);
+    a.oct_h = dalloc<float4>(d_allocs_, noct);
+    a.oct_c2 = full_ ? dalloc<float4>(d_allocs_, noct) : nullptr;
+    a.oct_h2 = full_ ? dalloc<float4>(d_allocs_, noct) : nullptr;
     a.hb_c = dalloc<float4>(d_allocs_, 2 * (size_t)NB_);
     a.hb_h = dalloc<float4>(d_allocs_, 2 * (size_t)NB_);
     a.hb_c2 = full_ ? dalloc<float4>(d_allocs_, 2 * (size_t)NB_) : nullptr;

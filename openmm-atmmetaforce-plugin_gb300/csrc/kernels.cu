@@ -42,10 +42,10 @@ __device__ __forceinline__ float wrapf(float x, float L, float iL) { return x - 
 // prepare: one warp per block
 // ---------------------------------------------------------------------------
 // Bounding box of a block (minimum image relative to its first atom); h.w receives
-// the number of real (non-padding) atoms of the block.  With hc, also the boxes of its
+// the number of real (non-padding) atoms of the block; box: c and h again.  With hc, also the boxes of its
 // two halves, whose h.w receives the largest distance of an atom from the box centre.
 __device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDev& R, int b, float4* c, float4* h,
-                                          float4* hc, float4* hh, int lane, int nreal) {
+                                          float4* hc, float4* hh, int lane, int nreal, float4* box) {
     float x0 = __shfl_sync(FULL_MASK, x, 0), y0 = __shfl_sync(FULL_MASK, y, 0), z0 = __shfl_sync(FULL_MASK, z, 0);
     float dx = x - x0, dy = y - y0, dz = z - z0;
     min_image3(dx, dy, dz, R);
@@ -71,8 +71,35 @@ __device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDe
         hz = fmaxf(hz, __shfl_xor_sync(FULL_MASK, hz, o));
     }
     if (lane == 0) {
-        c[b] = make_float4(x0 + 0.5f * (lx + hx), y0 + 0.5f * (ly + hy), z0 + 0.5f * (lz + hz), 0.f);
-        h[b] = make_float4(0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz), __int_as_float(nreal));
+        c[b] = box[0] = make_float4(x0 + 0.5f * (lx + hx), y0 + 0.5f * (ly + hy), z0 + 0.5f * (lz + hz), 0.f);
+        h[b] = box[1] = make_float4(0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz), __int_as_float(nreal));
+    }
+}
+
+// The box around the eight blocks of a CTA (one warp; box: their centres and half
+// extents, rep: their replicas, -1: none), at the images nearest the first one's centre.
+__device__ __forceinline__ void octet_bbox(const Args& a, const float4 (*box)[2], const int* rep, int lane, float4* c,
+                                           float4* h) {
+    const RepDev& R = a.reps[rep[0]];
+    const int k = rep[lane & 7] < 0 ? 0 : lane & 7;
+    const bool mixed = __any_sync(FULL_MASK, rep[k] != rep[0]) || R.tric;
+    const float4 c0 = box[0][0], cb = box[k][0], hb = box[k][1];
+    float dx = cb.x - c0.x, dy = cb.y - c0.y, dz = cb.z - c0.z;
+    min_image3(dx, dy, dz, R);
+    float lx = dx - hb.x, ly = dy - hb.y, lz = dz - hb.z, hx = dx + hb.x, hy = dy + hb.y, hz = dz + hb.z;
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1) {
+        lx = fminf(lx, __shfl_xor_sync(FULL_MASK, lx, o));
+        ly = fminf(ly, __shfl_xor_sync(FULL_MASK, ly, o));
+        lz = fminf(lz, __shfl_xor_sync(FULL_MASK, lz, o));
+        hx = fmaxf(hx, __shfl_xor_sync(FULL_MASK, hx, o));
+        hy = fmaxf(hy, __shfl_xor_sync(FULL_MASK, hy, o));
+        hz = fmaxf(hz, __shfl_xor_sync(FULL_MASK, hz, o));
+    }
+    if (lane == 0) {
+        *c = make_float4(c0.x + 0.5f * (lx + hx), c0.y + 0.5f * (ly + hy), c0.z + 0.5f * (lz + hz), 0.f);
+        *h = mixed ? make_float4(1e30f, 1e30f, 1e30f, 0.f)
+                   : make_float4(0.5f * (hx - lx), 0.5f * (hy - ly), 0.5f * (hz - lz), 0.f);
     }
 }
 
@@ -97,7 +124,7 @@ __device__ __forceinline__ void decide_build(const Args& a) {
     if (build) a.list_counts[1]++;
 }
 
-constexpr int kPrepThreads = 256;
+constexpr int kPrepThreads = 256;  // (eight blocks: an octet of the finder)
 
 // CTAs below nprep prepare eight blocks each; the rest zero the int32 charge grids,
 // which the spreading adds into (a memset node of its own cost the PME chain its
@@ -112,8 +139,11 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
             g[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
+    __shared__ float4 s_box[2][kPrepThreads / 32][2];
+    __shared__ int s_rep[kPrepThreads / 32];
     int lane = threadIdx.x & 31;
     int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (lane == 0) s_rep[threadIdx.x >> 5] = b < a.NB ? a.block_rep[b] : -1;
     if (b < a.NB) {
         int s = b * kTile + lane;
         int rep = a.block_rep[b];
@@ -152,7 +182,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
         for (int k = 0; k < 6; k++) a.F[(size_t)k * a.NA + s] = 0ull;
         if (a.adjoint)
             for (int k = 0; k < 3; k++) a.D[(size_t)k * a.NA + s] = 0ull;
-        warp_bbox(x, y, z, R, b, a.bb_c, a.bb_h, a.any_tric ? a.hb_c : nullptr, a.hb_h, lane, nreal);
+        warp_bbox(x, y, z, R, b, a.bb_c, a.bb_h, a.any_tric ? a.hb_c : nullptr, a.hb_h, lane, nreal,
+                  s_box[0][threadIdx.x >> 5]);
         if (R.tric && lane == 0) {  // (lane 0 wrote the box)
             const float4 h = a.bb_h[b];
             atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));
@@ -163,15 +194,19 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
             wrap3(x2, y2, z2, R);
             a.posq2[s] = make_float4(x2, y2, z2, q);
             warp_bbox(x2, y2, z2, R, b, a.bb_c2, a.bb_h2, a.any_tric ? a.hb_c2 : nullptr, a.hb_h2, lane,
-                      nreal);
+                      nreal, s_box[1][threadIdx.x >> 5]);
             if (R.tric && lane == 0) {
                 const float4 h = a.bb_h2[b];
                 atomicMax(&a.rep_hmax[rep], __float_as_uint(sqrtf(h.x * h.x + h.y * h.y + h.z * h.z)));
             }
         }
     }
+    __syncthreads();  // the boxes; with a skin, this CTA's maxima precede its count
+    if (threadIdx.x < 32)
+        octet_bbox(a, s_box[0], s_rep, lane, &a.oct_c[blockIdx.x], &a.oct_h[blockIdx.x]);
+    else if (threadIdx.x < 64 && a.full)
+        octet_bbox(a, s_box[1], s_rep, lane, &a.oct_c2[blockIdx.x], &a.oct_h2[blockIdx.x]);
     if (a.skin_half2 > 0.f) {
-        __syncthreads();  // this CTA's maxima precede its count
         if (threadIdx.x == 0) {
             __threadfence();
             if (atomicAdd(&a.status->prepared, 1) == nprep - 1) {

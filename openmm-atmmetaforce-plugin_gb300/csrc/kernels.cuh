@@ -250,6 +250,8 @@ struct Args {
     float4* bb_h;             // NB: half extents
     float4* bb_c2;            // NB: state 2 (full mode)
     float4* bb_h2;
+    float4 *oct_c, *oct_h;    // ceil(NB / 8): box of blocks 8 o .. 8 o + 7 (without limits where they
+    float4 *oct_c2, *oct_h2;  //   belong to two replicas or the box is triclinic); state 2
     float4 *hb_c, *hb_h;      // 2 NB: the same of the half blocks (triclinic batches; h.w: radius
     float4 *hb_c2, *hb_h2;    //   about the centre)
     // rows and tiles

@@ -231,53 +231,57 @@ __device__ __forceinline__ int exact_cut_half(const Args& a, const RepDev& R, in
     const float rcm = sqrtf(a.rcl2) + kHalfCutMargin;
     const __half2 thr = __float2half2_rn(rcm * rcm);
     const uint4* ih = reinterpret_cast<const uint4*>(s_ipos);
+    const unsigned lt = (1u << lane) - 1u;
+    // atoms per lane, which share each i atom's read (1 / 2 / 3: 163 / 159 / 161 M warp
+    // instructions, 254 / 244 / 251 us on 22 x 23,558 atoms; 170 M and 258 us with a
+    // comparison per pair and an exit when every lane had a hit)
+    constexpr int kPer = 2;
     int kept = from;
-    for (int g = from; g < natom; g += 32) {
-        const int k = g + lane;
-        const bool valid = k < natom;
-        const int j = valid ? list[k] : 0;
-        float rx = 64.f, ry = 64.f, rz = 64.f;  // invalid lanes never hit
-        if (valid) {
-            const float4 p = row_pos(a, kind, j);
-            rx = p.x - ci.x;
-            ry = p.y - ci.y;
-            rz = p.z - ci.z;
+    for (int g = from; g < natom; g += 32 * kPer) {
+        int j[kPer];
+        bool valid[kPer];
+        __half2 hx[kPer], hy[kPer], hz[kPer], least[2][kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            valid[u] = g + 32 * u + lane < natom;
+            j[u] = list[valid[u] ? g + 32 * u + lane : g];
+        }
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const float4 p = row_pos(a, kind, j[u]);
+            float rx = p.x - ci.x, ry = p.y - ci.y, rz = p.z - ci.z;
             min_image_t<TRIC>(rx, ry, rz, R);
+            hx[u] = __float2half2_rn(rx);
+            hy[u] = __float2half2_rn(ry);
+            hz[u] = __float2half2_rn(rz);
         }
-        const __half2 hx = __float2half2_rn(rx), hy = __float2half2_rn(ry), hz = __float2half2_rn(rz);
-        bool hitA = false, hitB = false;
-        // two i atoms per instruction, eight per step; each half until every lane has decided it
-        for (int m0 = 0; m0 < kHalf / 2; m0 += 4) {
+        // two i atoms per instruction: the least squared distance to each half
 #pragma unroll
-            for (int m = m0; m < m0 + 4; m++) {
-                const uint4 q = ih[m];
-                const __half2 dx = __hsub2(hx, *reinterpret_cast<const __half2*>(&q.x));
-                const __half2 dy = __hsub2(hy, *reinterpret_cast<const __half2*>(&q.y));
-                const __half2 dz = __hsub2(hz, *reinterpret_cast<const __half2*>(&q.z));
-                const __half2 r2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
-                hitA |= !__hbge2(r2, thr);  // either atom of the pair within the widened cutoff
-            }
-            if (__all_sync(FULL_MASK, hitA || !valid)) break;
-        }
-        for (int m0 = kHalf / 2; m0 < kHalf; m0 += 4) {
+        for (int h = 0; h < 2; h++) {
 #pragma unroll
-            for (int m = m0; m < m0 + 4; m++) {
-                const uint4 q = ih[m];
-                const __half2 dx = __hsub2(hx, *reinterpret_cast<const __half2*>(&q.x));
-                const __half2 dy = __hsub2(hy, *reinterpret_cast<const __half2*>(&q.y));
-                const __half2 dz = __hsub2(hz, *reinterpret_cast<const __half2*>(&q.z));
-                const __half2 r2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
-                hitB |= !__hbge2(r2, thr);
+            for (int u = 0; u < kPer; u++) least[h][u] = __float2half2_rn(60000.0f);
+#pragma unroll
+            for (int m = 0; m < kHalf / 2; m++) {
+                const uint4 q = ih[h * (kHalf / 2) + m];
+#pragma unroll
+                for (int u = 0; u < kPer; u++) {
+                    const __half2 dx = __hsub2(hx[u], *reinterpret_cast<const __half2*>(&q.x));
+                    const __half2 dy = __hsub2(hy[u], *reinterpret_cast<const __half2*>(&q.y));
+                    const __half2 dz = __hsub2(hz[u], *reinterpret_cast<const __half2*>(&q.z));
+                    // (a distance that is no number stays and counts as a hit)
+                    least[h][u] = __hmin2_nan(least[h][u], __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz))));
+                }
             }
-            if (__all_sync(FULL_MASK, hitB || !valid)) break;
         }
         __syncwarp();
-        const bool keep = valid && (hitA || hitB);
-        const unsigned b = __ballot_sync(FULL_MASK, keep);
-        if (keep)
-            list[kept + __popc(b & ((1u << lane) - 1u))] =
-                (int)((unsigned)j | (hitA ? kHalfA : 0u) | (hitB ? kHalfB : 0u));
-        kept += __popc(b);
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const bool hitA = valid[u] && !__hbge2(least[0][u], thr), hitB = valid[u] && !__hbge2(least[1][u], thr);
+            const unsigned b = __ballot_sync(FULL_MASK, hitA || hitB);
+            if (hitA || hitB)
+                list[kept + __popc(b & lt)] = (int)((unsigned)j[u] | (hitA ? kHalfA : 0u) | (hitB ? kHalfB : 0u));
+            kept += __popc(b);
+        }
         __syncwarp();
     }
     return kept;
@@ -345,6 +349,13 @@ __device__ __noinline__ int exact_cut(const Args& a, const RepDev& R, int kind, 
 // The row's exclusion partners are held one per lane (rows with more than 32 fall
 // back to reading the list), and four candidate blocks are loaded per step so
 // that their latencies overlap.
+//
+// Which blocks are tested: rows in one part first test the boxes of octets of blocks
+// (consecutive along the Hilbert curve, so compact), 32 at once, and then the blocks of
+// the octets within the cutoff, four octets at once; rows in parts test their blocks in
+// strides, 32 at once.  Bound by instruction issue (62 % active): octets take 22 x
+// 23,558 atoms from 159 to 148 M warp instructions, and the candidate tests off the time
+// of long rows: 8 x 60,000 atoms 311 -> 216 us, 22 x 23,558 244 -> 238.
 template <bool CUT, bool TRIC>
 __device__ __forceinline__ int row_atoms(const Args& a, const RepDev& R, int I, int kind, float4 ci, float4 hi,
                                          const int2* ee, int e0, int e1, int lane, int* out, int cap,
@@ -354,16 +365,49 @@ __device__ __forceinline__ int row_atoms(const Args& a, const RepDev& R, int I, 
     const bool g2 = kind == ROW_DIFF2;
     const int cls_i = a.block_cls[I];
     const float4* P = kind == ROW_STATE2 ? a.posq2 : a.posq;
-    const float4* BH = kind == ROW_STATE2 ? a.bb_h2 : a.bb_h;
     const int nex = e1 - e0;
     const int my_ex = lane < nex ? ee[e0 + lane].x : -1;
     int natom = 0, cut_from = 0;
     bool over = false;
     raw = 0;
     const int jb = diff ? R.block_begin : I + 1;
-    for (int base = jb + first; base < R.block_end; base += 32 * stride) {
-        const int Jl = base + lane * stride;
-        bool ok = Jl < R.block_end;
+    const float4* OC = kind == ROW_STATE2 ? a.oct_c2 : a.oct_c;
+    const float4* OH = kind == ROW_STATE2 ? a.oct_h2 : a.oct_h;
+    unsigned octs = 0u;  // octets from ob on still to be taken
+    int ob = 0;
+    for (int base = stride > 1 ? jb + first : jb & ~7; octs || base < R.block_end;) {
+        int Jl;
+        if (stride > 1) {
+            Jl = base + lane * stride;
+            base += 32 * stride;
+        } else {
+            if (!octs) {
+                ob = base >> 3;
+                base += 256;
+                const int o = ob + lane;
+                bool near = 8 * o < R.block_end;
+                if (near && !(g2 && 8 * o + 8 > R.mov_block_begin)) {  // (moving blocks are displaced)
+                    const float4 co = OC[o], ho = OH[o];
+                    float dx = co.x - ci.x, dy = co.y - ci.y, dz = co.z - ci.z;
+                    min_image_t<TRIC>(dx, dy, dz, R);
+                    near = !(box_gap2(dx, dy, dz, hi.x + ho.x, hi.y + ho.y, hi.z + ho.z) >= a.rcl2 * 1.0001f);
+                }
+                octs = __ballot_sync(FULL_MASK, near);
+                if (!octs) continue;
+            }
+            // the lowest four octets, eight lanes each
+            int o = __ffs(octs) - 1;
+            octs &= octs - 1;
+#pragma unroll
+            for (int q = 1; q < 4; q++) {
+                const int oq = octs ? __ffs(octs) - 1 : -1;
+                octs &= octs - 1;
+                if ((lane >> 3) == q) o = oq;
+            }
+            Jl = o >= 0 ? 8 * (ob + o) + (lane & 7) : R.block_end;
+        }
+        int nl = 0;  // atoms of this lane's block
+        bool ok = Jl < R.block_end && Jl >= jb;
         if (ok && diff) {
             const int cj = a.block_cls[Jl];
             ok = Jl != I && cj != cls_i && (cj == 0 || cls_i < cj);
@@ -384,6 +428,7 @@ __device__ __forceinline__ int row_atoms(const Args& a, const RepDev& R, int I, 
                 }
             }
             ok = boxes_close<TRIC>(ci, hi, cj4, hj4, R, a.rcl2, all_images);
+            nl = __float_as_int(hj4.w);
             if (nex > 32)
                 for (int k = e0; ok && k < e1; k++)
                     if (ee[k].x == Jl) ok = false;
@@ -401,19 +446,23 @@ __device__ __forceinline__ int row_atoms(const Args& a, const RepDev& R, int I, 
             float4 p[4];
 #pragma unroll
             for (int t = 0; t < 4; t++) {
-                J[t] = cand ? base + (__ffs(cand) - 1) * stride : -1;
-                if (cand) cand &= cand - 1;
+                const int src = (__ffs(cand) - 1) & 31;  // (none left: any block, no atoms)
+                J[t] = __shfl_sync(FULL_MASK, Jl, src);
+                n[t] = __shfl_sync(FULL_MASK, nl, src);
+                if (!cand) {
+                    J[t] = J[0];
+                    n[t] = 0;
+                }
+                cand &= cand - 1;
             }
 #pragma unroll
             for (int t = 0; t < 4; t++) {
-                const int jj = (J[t] >= 0 ? J[t] : J[0]) * kTile + lane;
-                p[t] = P[jj];
-                n[t] = J[t] >= 0 ? __float_as_int(BH[J[t]].w) : 0;
+                p[t] = P[J[t] * kTile + lane];
             }
             if (g2) {
 #pragma unroll
                 for (int t = 0; t < 4; t++) {
-                    const float4 d = a.displ[(J[t] >= 0 ? J[t] : J[0]) * kTile + lane];
+                    const float4 d = a.displ[J[t] * kTile + lane];
                     p[t].x += d.x;
                     p[t].y += d.y;
                     p[t].z += d.z;
@@ -425,22 +474,29 @@ __device__ __forceinline__ int row_atoms(const Args& a, const RepDev& R, int I, 
                 const bool in = lane < n[t] && (all_images || point_close<TRIC>(ci, hi, p[t], R, a.rcl2));
                 const unsigned b = __ballot_sync(FULL_MASK, in);
                 const int k = natom + __popc(b & ((1u << lane) - 1u));
-                if (in && k < cap && !over) out[k] = J[t] * kTile + lane;
+                // (with the cut, four blocks always fit)
+                if (in && (CUT ? !over : k < cap)) out[k] = J[t] * kTile + lane;
                 natom += __popc(b);
-                raw += __popc(b);
             }
             if (CUT && !over && natom > cap - 4 * kTile) {
                 __syncwarp();
-                natom = exact_cut<TRIC>(a, R, kind, ci, lane, out, cut_from, min(natom, cap), s_ipos, hcut);
+                const int before = natom;
+                natom = exact_cut<TRIC>(a, R, kind, ci, lane, out, cut_from, natom, s_ipos, hcut);
+                raw += before - natom;
                 cut_from = natom;
                 over = natom > cap - 4 * kTile;
             }
         }
     }
     if (CUT) {
-        if (over) return -1;
+        if (over) {
+            raw += natom;
+            return -1;
+        }
         __syncwarp();
         natom = exact_cut<TRIC>(a, R, kind, ci, lane, out, cut_from, natom, s_ipos, hcut);
+    } else {
+        raw = natom;
     }
     return natom;
 }

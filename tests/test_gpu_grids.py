@@ -126,3 +126,26 @@ def test_triclinic_rows_by_groups(n, L, ligand, diff):
     ref = O.atm_eval(c.spec, c.pos, c.displ, c.params)
     assert abs(r[0]["pert"] - ref["usc"]) <= U_TOL
     assert np.sqrt(((F - ref["forces"]) ** 2).sum() / (ref["forces"] ** 2).sum()) <= F_TOL
+
+
+@pytest.mark.parametrize("atoms", [(1103, 2207, 1500), (9001, 1103)])
+def test_octets_of_blocks_across_replicas(atoms):
+    """Octets that belong to two replicas, that hold the last blocks of one, moving blocks
+    at their displaced positions, and rows in one part (enough replicas) and in several,
+    against batches of one replica."""
+    cases = [S.water_ligand_box(n, (n / 98.85) ** (1 / 3), [9 + k], [(0.9, 1.0, 0.8)], S.PME, 0.9, seed=130 + k)
+             for k, n in enumerate(atoms)]
+    many = [cases[k % len(cases)] for k in range(48 if len(atoms) == 3 else 2)]
+    for diff in (0, 1):
+        one = [atm.ReplicaBatch([atm.system_from_case(c)[0]], 0, {"DifferencePath": diff}) for c in cases]
+        want = [b.evaluate(c.pos, as_array=True) for b, c in zip(one, cases)]
+        systems = [atm.system_from_case(c)[0] for c in cases]
+        b = atm.ReplicaBatch([systems[k % len(cases)] for k in range(len(many))], 0, {"DifferencePath": diff})
+        E, F, r = b.evaluate(np.concatenate([c.pos for c in many]), as_array=True)
+        for k in range(len(many)):
+            e, f, q = want[k % len(cases)]
+            got = F[b.offsets[k]:b.offsets[k + 1]]
+            # rows in another number of parts group their pairs otherwise: FP32 sums of at
+            # most 16 terms, a few 2^-24 of the pair forces
+            assert np.sqrt(((got - f) ** 2).sum() / (f ** 2).sum()) <= 2e-6, (diff, k)
+            assert abs(r[k][atm.RES_KEYS.index("u")] - q[0][atm.RES_KEYS.index("u")]) <= U_TOL
