@@ -449,21 +449,24 @@ struct Stencil {
     float dw[3][5];
 };
 
+// One dimension of a stencil at fractional coordinate f of K grid points: the top
+// point's index, weights and derivatives.
+__device__ __forceinline__ int stencil_dim(float f, int K, float* w, float* dw) {
+    f -= floorf(f);
+    float u = f * (float)K;
+    int b = (int)floorf(u);
+    float t = u - (float)b;
+    if (b >= K) b -= K;
+    if (b < 0) b += K;
+    bspline5(t, w, dw);
+    return b;
+}
+
 __device__ __forceinline__ void make_stencil(float x, float y, float z, const RepDev& R, Stencil& S, bool deriv) {
     float fr[3];
     frac3(x, y, z, R, fr);
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        float f = fr[d];
-        f -= floorf(f);
-        float u = f * (float)R.K[d];
-        int b = (int)floorf(u);
-        float t = u - (float)b;
-        if (b >= R.K[d]) b -= R.K[d];
-        if (b < 0) b += R.K[d];
-        S.base[d] = b;
-        bspline5(t, S.w[d], deriv ? S.dw[d] : nullptr);
-    }
+    for (int d = 0; d < 3; d++) S.base[d] = stencil_dim(fr[d], R.K[d], S.w[d], deriv ? S.dw[d] : nullptr);
 }
 
 // Charge spreading by bricks.  One CTA holds one brick (the tuned edge, 12 to 20
@@ -769,6 +772,7 @@ static_assert(kExcThreads == kSpreadAtomWarps * 32, "exceptions and spreading sh
 
 __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a, int nexc) {
     __shared__ float s_st[kSpreadAtomWarps][kSpreadAtoms * kStencilWords];
+    __shared__ int s_base[kSpreadAtomWarps][3][kSpreadAtoms];
     if ((int)blockIdx.x < nexc) {
         exceptions_cta(a, blockIdx.x);
         return;
@@ -788,8 +792,12 @@ __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a, 
         code = (m & 1) ? 3 : 1;
     }
     const RepDev& R = a.reps[a.block_rep[blk]];
-    const int at = part * kSpreadAtoms + lane;  // atom of the block (lanes below kSpreadAtoms)
-    const int s = blk * kTile + (min(at, kTile - 1));
+    const int K0 = R.K[0], K1 = R.K[1], K2 = R.K[2];
+    // one dimension of one atom's stencil per lane: lane 8 d + t, dimension d (lanes 24
+    // and beyond repeat the last)
+    const int t = lane & (kSpreadAtoms - 1), d = min(lane / kSpreadAtoms, 2);
+    const int at = part * kSpreadAtoms + t;  // atom of the block
+    const int s = blk * kTile + at;
     const int nreal = __float_as_int(a.bb_h[blk].w);
     float4 p = a.posq[s];
     if (code == 1) p.w = -p.w;
@@ -800,42 +808,39 @@ __global__ void __launch_bounds__(kSpreadAtomWarps * 32) k_spread_atoms(Args a, 
         p.z += dd.z;
         wrap3(p.x, p.y, p.z, R);
     }
-    const bool ok = lane < kSpreadAtoms && at < nreal && p.w != 0.0f;
+    const bool ok = at < nreal && p.w != 0.0f;
     float* st = s_st[w];
-    if (ok) {
-        Stencil S;
-        make_stencil(p.x, p.y, p.z, R, S, false);
-        float* wv = st + lane * kStencilWords;
+    if (ok && lane < 3 * kSpreadAtoms) {
+        float fr[3], ws[kOrder];
+        frac3(p.x, p.y, p.z, R, fr);
+        const int b = stencil_dim(d == 0 ? fr[0] : d == 1 ? fr[1] : fr[2], d == 0 ? K0 : d == 1 ? K1 : K2, ws, nullptr);
+        float* wv = st + t * kStencilWords + d * kOrder;
         const float qs = p.w * kGridScale;
 #pragma unroll
-        for (int k = 0; k < kOrder; k++) {
-            wv[k] = qs * S.w[0][k];
-            wv[kOrder + k] = S.w[1][k];
-            wv[2 * kOrder + k] = S.w[2][k];
-        }
-        wv[15] = __int_as_float((S.base[0] << 20) | (S.base[1] << 10) | S.base[2]);
+        for (int k = 0; k < kOrder; k++) wv[k] = d == 0 ? qs * ws[k] : ws[k];
+        s_base[w][d][t] = b;
     }
-    unsigned bal = __ballot_sync(FULL_MASK, ok);
+    unsigned bal = __ballot_sync(FULL_MASK, ok && lane < kSpreadAtoms);
     __syncwarp();
-    const int K0 = R.K[0], K1 = R.K[1], K2 = R.K[2];
     int* G = reinterpret_cast<int*>(a.qreal + R.real_off + (code ? (size_t)K0 * K1 * K2 : 0));
     const int b0 = lane / kOrder, c0 = lane % kOrder;
     if (lane >= kOrder * kOrder) return;
+    const int plane = K1 * K2, wrap0 = K0 * plane;  // (a grid has fewer than 2^30 points)
     while (bal) {
         const int src = __ffs(bal) - 1;
         bal &= bal - 1;
         const float* wv = st + src * kStencilWords;
-        const int bases = __float_as_int(wv[15]);
-        int y = ((bases >> 10) & 1023) - b0, z = (bases & 1023) - c0;
+        int y = s_base[w][1][src] - b0, z = s_base[w][2][src] - c0;
         y += y < 0 ? K1 : 0;
         z += z < 0 ? K2 : 0;
         const float wyz = wv[kOrder + b0] * wv[2 * kOrder + c0];
-        const int x0 = bases >> 20;
+        int x = s_base[w][0][src] * plane;
+        int* row = G + y * K2 + z;
 #pragma unroll
         for (int a0 = 0; a0 < kOrder; a0++) {
-            int x = x0 - a0;
-            x += x < 0 ? K0 : 0;
-            atomicAdd(G + ((size_t)x * K1 + y) * K2 + z, __float2int_rn(wv[a0] * wyz));
+            atomicAdd(row + x, __float2int_rn(wv[a0] * wyz));
+            x -= plane;
+            x += x < 0 ? wrap0 : 0;
         }
     }
 }
