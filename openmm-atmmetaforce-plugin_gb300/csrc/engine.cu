@@ -275,7 +275,8 @@ Engine::~Engine() {
 void Engine::destroy_graphs() {
     if (graph_dev_) cudaGraphExecDestroy(graph_dev_);
     if (graph_res_) cudaGraphExecDestroy(graph_res_);
-    graph_dev_ = graph_res_ = nullptr;
+    if (graph_lean_) cudaGraphExecDestroy(graph_lean_);
+    graph_dev_ = graph_res_ = graph_lean_ = nullptr;
 }
 
 void Engine::set_positions(int r, const double* pos) {
@@ -1297,7 +1298,7 @@ void Engine::alloc_device() {
     }
     a.e_self = dupload(d_allocs_, e_self_);
     a.ends = dalloc<double>(d_allocs_, 2 * (size_t)R_);
-    a.merge_w = dalloc<double>(d_allocs_, (size_t)R_);
+    a.merge_w = dalloc<long long>(d_allocs_, (size_t)R_);
     a.results = dalloc<double>(d_allocs_, (size_t)R_ * NUM_RES);
     a.matrix = dalloc<double>(d_allocs_, (size_t)R_ * R_);
     a.beta = reinterpret_cast<double*>(d_params_ + 40);
@@ -1394,7 +1395,7 @@ void Engine::upload_params(cudaStream_t st) {
 // One evaluation: kernels only (the parameter block is uploaded before the graph when
 // it changed, the grids are zeroed by k_prepare and the host's copies written by the
 // last kernels).
-void Engine::record(cudaStream_t st, const Args& a) {
+void Engine::record(cudaStream_t st, const Args& a, bool output) {
     launch_prepare(a, st);
     bool pme = method_ == NonbondedForce::PME;
     if (pme) {
@@ -1422,7 +1423,21 @@ void Engine::record(cudaStream_t st, const Args& a) {
     if (!pme) launch_exceptions(a, st);
     if (pme && tune_pme_stream_) CUDA_CHECK(cudaStreamWaitEvent(st, ev_join_, 0));
     launch_finalize(a, st);
-    launch_output(a, st);
+    if (output) launch_output(a, st);
+}
+
+void Engine::capture(cudaGraphExec_t& gx, const Args& a, bool output) {
+    cudaGraph_t g;
+    CUDA_CHECK(cudaStreamBeginCapture(s_main_, cudaStreamCaptureModeThreadLocal));
+    try {
+        record(s_main_, a, output);
+    } catch (...) {
+        cudaStreamEndCapture(s_main_, &g);
+        throw;
+    }
+    CUDA_CHECK(cudaStreamEndCapture(s_main_, &g));
+    CUDA_CHECK(cudaGraphInstantiate(&gx, g, cudaGraphInstantiateFlagUseNodePriority));
+    CUDA_CHECK(cudaGraphDestroy(g));
 }
 
 // Charge grids -> potential grids: the hand-written transforms with the
@@ -1543,19 +1558,7 @@ void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos_pin
             times_.erase(times_.begin());
         } else {
             cudaGraphExec_t& gx = a.h_results ? graph_res_ : graph_dev_;
-            if (!gx) {
-                cudaGraph_t g;
-                CUDA_CHECK(cudaStreamBeginCapture(s_main_, cudaStreamCaptureModeThreadLocal));
-                try {
-                    record(s_main_, a);
-                } catch (...) {
-                    cudaStreamEndCapture(s_main_, &g);
-                    throw;
-                }
-                CUDA_CHECK(cudaStreamEndCapture(s_main_, &g));
-                CUDA_CHECK(cudaGraphInstantiate(&gx, g, cudaGraphInstantiateFlagUseNodePriority));
-                CUDA_CHECK(cudaGraphDestroy(g));
-            }
+            if (!gx) capture(gx, a, true);
             CUDA_CHECK(cudaGraphLaunch(gx, st));
             CUDA_CHECK(cudaStreamSynchronize(st));
         }
@@ -1657,7 +1660,7 @@ void Engine::run_device(const double* d_pos, cudaStream_t stream) {
     run(stream, d_pos);
 }
 
-void Engine::launch_device(const double* d_pos, cudaStream_t stream) {
+void Engine::launch_device(const double* d_pos, cudaStream_t stream, bool output) {
     CUDA_CHECK(cudaSetDevice(dev_));
     if (!layout_ready_ || force_build_ || !graph_dev_) {
         // a new layout, new buffers or a forced build: the synchronous path (it
@@ -1677,7 +1680,8 @@ void Engine::launch_device(const double* d_pos, cudaStream_t stream) {
         CUDA_CHECK(cudaMemcpyAsync((void*)A_.pos_in, d_pos, sizeof(double) * 3 * (size_t)n_in_,
                                    cudaMemcpyDeviceToDevice, stream));
     upload_params(stream);
-    CUDA_CHECK(cudaGraphLaunch(graph_dev_, stream));
+    if (!output && !graph_lean_) capture(graph_lean_, A_, false);
+    CUDA_CHECK(cudaGraphLaunch(output ? graph_dev_ : graph_lean_, stream));
 }
 
 void Engine::set_position_source(const double* d_pos) {

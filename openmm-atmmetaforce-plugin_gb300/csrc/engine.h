@@ -99,7 +99,11 @@ public:
     // poll_overflow() before it trusts a result that a list build overflowed
     // (builds happen at the evaluations where atoms have moved beyond half the
     // skin, or when forced).
-    void launch_device(const double* d_pos, cudaStream_t stream);
+    // output = false: without the force output, the result records and the matrix (the
+    // caller takes the merged forces from device_args(): F, slot_of, merge_w); the status
+    // that poll_overflow() reads is that of the last evaluation with output.
+    void launch_device(const double* d_pos, cudaStream_t stream, bool output = true);
+    const Args& device_args() const { return A_; }
     // After a synchronisation of the stream of the evaluations: true if a list
     // build since the last poll overflowed its capacity (the capacities are then
     // grown and the next evaluation builds the lists again; the results of the
@@ -168,7 +172,8 @@ private:
     void update_rep_table();
     double dispersion_energy(int r);
     double self_factor() const;
-    void record(cudaStream_t main, const Args& a);
+    void record(cudaStream_t main, const Args& a, bool output);
+    void capture(cudaGraphExec_t& gx, const Args& a, bool output);
     void pme_transforms(cudaStream_t st, const std::function<void(const char*)>& mark = nullptr);
     // The device mirror of the parameter block, brought up to date on the stream.
     void upload_params(cudaStream_t st);
@@ -292,7 +297,8 @@ private:
 
     cudaStream_t s_main_ = nullptr, s_pme_ = nullptr;
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
-    cudaGraphExec_t graph_dev_ = nullptr, graph_res_ = nullptr;  // without / with host results
+    // without and with host results; without any output
+    cudaGraphExec_t graph_dev_ = nullptr, graph_res_ = nullptr, graph_lean_ = nullptr;
     std::vector<KernelTime> times_;
 };
 

@@ -1345,7 +1345,7 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(Args a) {
         a.ends[2 * r + 1] = E2;
         // a NonbondedForce outside the variable groups contributes nothing to U_var
         const MergeHead m = merge_head(R.var_nb ? E1 : 0.0, R.var_nb ? E2 : 0.0, R.params);
-        a.merge_w[r] = R.params[8] > 0 ? m.sp : 1.0 - m.sp;
+        a.merge_w[r] = __double2ll_rn((R.params[8] > 0 ? m.sp : 1.0 - m.sp) * 4294967296.0);
         a.rep_hmax[r] = 0u;  // ready for the next evaluation (the finder has read it)
     }
 }
@@ -1419,20 +1419,13 @@ __global__ void __launch_bounds__(kOutThreads) k_output(Args a, int nmat) {
         const int s = a.slot_of[g];
         const int rep = a.block_rep[s >> 5];
         const RepDev& R = a.reps[rep];
-        const double wgt = a.merge_w[rep];
-        // F1 + w (F2 - F1) in the fixed point of the force sums, w in units of 2^-32
-        // (w in [0, 1]: at most 2^32; its rounding is 2^-33 relative to F2 - F1),
-        // the product by a 128-bit multiply (floor), then one conversion per
-        // component and the exact 2^-32 scaling in the exponent field
-        const long long w32 = __double2ll_rn(wgt * 4294967296.0);
+        // merged in fixed point, then one conversion per component and the exact 2^-32
+        // scaling in the exponent field
+        const long long w32 = a.merge_w[rep];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const long long f1 = (long long)a.F[(size_t)k * a.NA + s];
-            const long long f2 = (long long)a.F[(size_t)(3 + k) * a.NA + s];
-            const long long d = a.full ? f2 - f1 : f2;
-            const long long hi = __mul64hi(d, w32);
-            const unsigned long long lo = (unsigned long long)d * (unsigned long long)w32;
-            const long long v = f1 + (long long)(((unsigned long long)hi << 32) | (lo >> 32));
+            const long long v = merged_fix(f1, (long long)a.F[(size_t)(3 + k) * a.NA + s], a.full, w32);
             f[k] = R.var_nb ? fix_scaled(v) : 0.0;
             if (fnb) fb[k] = fix_scaled(f1);
         }

@@ -39,6 +39,16 @@ __device__ __forceinline__ double fix_scaled(long long v) {
     const double d = (double)v;
     return v == 0 ? 0.0 : __longlong_as_double(__double_as_longlong(d) - (32LL << 52));
 }
+
+// F1 + w (F2 - F1) in the fixed point of the force sums (f2: F2 - F1 already unless
+// full), w in units of 2^-32 (w in [0, 1]: at most 2^32; its rounding is 2^-33 relative
+// to F2 - F1), the product by a 128-bit multiply (floor).
+__device__ __forceinline__ long long merged_fix(long long f1, long long f2, int full, long long w32) {
+    const long long d = full ? f2 - f1 : f2;
+    const long long hi = __mul64hi(d, w32);
+    const unsigned long long lo = (unsigned long long)d * (unsigned long long)w32;
+    return f1 + (long long)(((unsigned long long)hi << 32) | (lo >> 32));
+}
 #endif
 
 // The z-row stride (words) of a spreading brick's int32 accumulator: at least n,
@@ -322,7 +332,7 @@ struct Args {
     // results
     double* e_self;           // R: PME self energies
     double* ends;             // R x 2: E1, E2
-    double* merge_w;          // R: the weight of F2 - F1 in the merged force
+    long long* merge_w;       // R: the weight of F2 - F1 in the merged force, units of 2^-32
     double* results;          // R * NUM_RES
     double* matrix;           // R * R
     const double* beta;       // device scalar

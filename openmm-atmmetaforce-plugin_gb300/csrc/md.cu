@@ -30,7 +30,13 @@ struct MdDev {
     const double* inv_m;
     const double* sqrt_inv_m;  // per atom, for the thermostat noise
     const int* rep_of;
-    const double* f_atm;
+    const double* f_atm;  // merged ATM forces (evaluations with output)
+    // ... and where the update takes them from (every evaluation)
+    const unsigned long long* F;
+    const int* slot_of;
+    const long long* merge_w;
+    const RepDev* reps;
+    int NA, full;
     unsigned long long* fb;
     double* e_terms;
     const MdBond* bonds;
@@ -216,9 +222,16 @@ __device__ __forceinline__ void md_integrate(const MdDev& a, int i, double* xn) 
     // FP64 is scarce on this part: per-atom factors once, then four fused
     // multiply-adds per component
     const double fim = a.fscale * im, nsim = a.noisescale * a.sqrt_inv_m[i];
+    // the merged ATM force straight from the fixed-point sums, as the evaluation's
+    // output kernel forms it (which most steps therefore do without)
+    const int s = a.slot_of[i];
+    const long long w32 = a.merge_w[r];
+    const bool var_nb = a.reps[r].var_nb;
     for (int k = 0; k < 3; k++) {
         size_t o = 3 * (size_t)i + k;
-        const double f = fma((double)(long long)a.fb[o], 1.0 / kFixScale, a.f_atm[o]);
+        const long long v1 = merged_fix((long long)a.F[(size_t)k * a.NA + s],
+                                        (long long)a.F[(size_t)(3 + k) * a.NA + s], a.full, w32);
+        const double f = fma((double)(long long)a.fb[o], 1.0 / kFixScale, var_nb ? fix_scaled(v1) : 0.0);
         const double v = fma(nsim, z[k], fma(fim, f, a.vscale * a.v[o]));
         xn[k] = fma(a.dt, v, a.x[o]);
     }
@@ -778,6 +791,13 @@ MdDev MDDriver::dev_args() const {
     a.sqrt_inv_m = sqrt_inv_m_;
     a.rep_of = rep_of_;
     a.f_atm = eng_->forces_device();
+    const Args& e = eng_->device_args();
+    a.F = e.F;
+    a.slot_of = e.slot_of;
+    a.merge_w = e.merge_w;
+    a.reps = e.reps;
+    a.NA = e.NA;
+    a.full = e.full;
     a.fb = fb_;
     a.e_terms = e_terms_;
     a.bonds = bonds_;
@@ -872,8 +892,12 @@ void MDDriver::set_recording(int interval, int capacity) {
 }
 
 // Device-to-device copies of the current evaluation into the ring (no host wait).
+bool MDDriver::record_due() const {
+    return rec_interval_ > 0 && step_ % rec_interval_ == 0 && step_ != rec_last_step_;
+}
+
 void MDDriver::record_step() {
-    if (rec_interval_ <= 0 || step_ % rec_interval_ != 0 || step_ == rec_last_step_) return;
+    if (!record_due()) return;
     const int slot = (int)(rec_count_ % rec_cap_);
     MD_CHECK(cudaMemcpyAsync(rec_res_ + (size_t)slot * R_ * NUM_RES, eng_->results_device(),
                              sizeof(double) * R_ * NUM_RES, cudaMemcpyDeviceToDevice, s_));
@@ -906,8 +930,10 @@ int MDDriver::get_records(long long* steps, double* results, double* matrices, i
 
 // The group-0 terms and the ATM evaluation at the current positions.  sync: wait
 // for the evaluation and grow the list capacities if a build overflowed (then
-// evaluate again); otherwise the evaluation is only enqueued.
-void MDDriver::compute_forces(bool sync) {
+// evaluate again); otherwise the evaluation is only enqueued.  output: with the force
+// output, records and status, which a step that is not recorded or checked does
+// without (the update merges the forces itself).
+void MDDriver::compute_forces(bool sync, bool output) {
     if (!have_positions_) throw Error(3, "Positions have not been set");
     MD_CHECK(cudaSetDevice(dev_));
     // the group-0 terms on their own stream, beside the ATM evaluation (after the
@@ -924,7 +950,7 @@ void MDDriver::compute_forces(bool sync) {
     }
     MD_CHECK(cudaEventRecord(ev_terms_, s_terms_));
     if (sync) eng_->run_device(x_, s_);  // synchronises and grows capacities as needed
-    else eng_->launch_device(x_, s_);
+    else eng_->launch_device(x_, s_, output);
     MD_CHECK(cudaStreamWaitEvent(s_, ev_terms_, 0));
     forces_valid_ = true;
 }
@@ -985,7 +1011,7 @@ void MDDriver::step(int nsteps) {
     snapshot();
     int since = 0;
     for (int k = 0; k < nsteps;) {
-        if (!forces_valid_) compute_forces(false);
+        if (!forces_valid_) compute_forces(false, record_due());
         record_step();
         MdDev a = dev_args();
         const int units = n_settle_ + n_cons_ + n_free_;

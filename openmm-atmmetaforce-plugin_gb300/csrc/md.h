@@ -124,7 +124,8 @@ public:
     const std::vector<int>& degrees_of_freedom() const { return dof_; }
 
 private:
-    void compute_forces(bool sync);
+    void compute_forces(bool sync, bool output = true);
+    bool record_due() const;
     void snapshot();
     void restore();
     bool check_lists();  // synchronises; true if steps since the snapshot must be redone
