@@ -39,7 +39,9 @@ struct atm_context_s {
     bool positions_set = false;
     bool dirty = true;
     double pert = 0.0;
-    std::vector<double> forces, forces_nb;
+    // the last evaluation's forces, summed over the groups asked for (held by the engine)
+    const double* forces = nullptr;
+    bool forces_atm = false, forces_nb = false;
     std::vector<double> results;
 };
 
@@ -613,8 +615,6 @@ int atm_context_create(atm_system_t sys, int device, const char* properties, atm
     c->eng->set_fused(prop_bool(props, "FusedTiles", false));
     c->eng->set_spread_owner(prop_bool(props, "SpreadByOwner", true));
     apply_spread_brick(*c->eng, props);
-    c->forces.resize(3 * (size_t)c->n);
-    c->forces_nb.resize(3 * (size_t)c->n);
     c->results.resize(NUM_RES);
     *out = c.release();
     API_END
@@ -671,9 +671,17 @@ int atm_context_get_state(atm_context_t ctx, int groups_mask, double* energy, do
     REQUIRE(ctx->positions_set, ATM_ERR_STATE, "Particle positions have not been set");
     bool want_atm = (groups_mask >> ctx->atm_group) & 1;
     bool want_nb = (groups_mask >> ctx->nb_group) & 1;
-    if ((want_atm || want_nb) && ctx->dirty) {
-        ctx->eng->evaluate(nullptr, ctx->forces.data(), ctx->forces_nb.data(), ctx->results.data(), nullptr);
-        ctx->dirty = false;
+    if (want_atm || want_nb) {
+        if (ctx->dirty) {
+            ctx->forces = ctx->eng->evaluate_forces(want_atm, want_nb, ctx->results.data());
+            ctx->dirty = false;
+            ctx->forces_atm = want_atm;
+            ctx->forces_nb = want_nb;
+        } else if (forces && (want_atm != ctx->forces_atm || want_nb != ctx->forces_nb)) {
+            ctx->forces = ctx->eng->output_forces(want_atm, want_nb);
+            ctx->forces_atm = want_atm;
+            ctx->forces_nb = want_nb;
+        }
     }
     // ATMMetaForceImpl.cpp:103,125: the perturbation energy is refreshed only when the ATM group is evaluated
     if (want_atm) ctx->pert = ctx->results[RES_PERT];
@@ -682,8 +690,9 @@ int atm_context_get_state(atm_context_t ctx, int groups_mask, double* energy, do
     if (want_nb) e += ctx->results[RES_E1];
     if (energy) *energy = e;
     if (forces) {
-        for (size_t k = 0; k < ctx->forces.size(); k++)
-            forces[k] = (want_atm ? ctx->forces[k] : 0.0) + (want_nb ? ctx->forces_nb[k] : 0.0);
+        const size_t bytes = sizeof(double) * 3 * (size_t)ctx->n;
+        if (want_atm || want_nb) std::memcpy(forces, ctx->forces, bytes);
+        else std::memset(forces, 0, bytes);
     }
     API_END
 }
@@ -770,7 +779,7 @@ int atm_batch_set_periodic_box_vectors(atm_batch_t b, int replica, const double*
 int atm_batch_evaluate(atm_batch_t b, const double* pos_all, double* energies, double* forces, double* results) {
     API_BEGIN
     REQUIRE(b, ATM_ERR_INVALID_ARGUMENT, "null batch");
-    b->eng->evaluate_host(pos_all, energies, forces, nullptr, b->results.data(), b->matrix.data());
+    b->eng->evaluate_host(pos_all, energies, forces, b->results.data(), b->matrix.data());
     if (results) std::memcpy(results, b->results.data(), sizeof(double) * b->results.size());
     b->evaluated = true;
     API_END

@@ -220,19 +220,18 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
     CUDA_CHECK(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
     CUDA_CHECK(cudaMallocHost(&h_pos_, sizeof(double) * 3 * (size_t)n_in_));
     CUDA_CHECK(cudaMallocHost(&h_forces_, sizeof(double) * 3 * (size_t)n_in_));
-    CUDA_CHECK(cudaMallocHost(&h_fnb_, sizeof(double) * 3 * (size_t)n_in_));
     CUDA_CHECK(cudaMallocHost(&h_results_, sizeof(double) * NUM_RES * (size_t)R_));
     CUDA_CHECK(cudaMallocHost(&h_matrix_, sizeof(double) * (size_t)R_ * R_));
-    // parameter block: ctl (2 ints) at 0, io (4 pointers) at 8, beta at 40, the
+    // parameter block: ctl (2 ints) at 0, io (3 pointers) at 8, beta at 32, the
     // replica table at kParamReps
     param_bytes_ = kParamReps + sizeof(RepDev) * (size_t)R_;
     CUDA_CHECK(cudaMallocHost(&h_params_, param_bytes_));
     std::memset(h_params_, 0, param_bytes_);
     h_ctl_ = reinterpret_cast<int*>(h_params_);
     h_io_ = reinterpret_cast<double**>(h_params_ + 8);
-    h_beta_ = reinterpret_cast<double*>(h_params_ + 40);
+    h_beta_ = reinterpret_cast<double*>(h_params_ + 32);
     h_reps_ = reinterpret_cast<RepDev*>(h_params_ + kParamReps);
-    for (int k = 0; k < 4; k++) h_io_[k] = nullptr;
+    for (int k = 0; k < 3; k++) h_io_[k] = nullptr;
     CUDA_CHECK(cudaMalloc(&d_counts_, 2 * sizeof(long long)));
     CUDA_CHECK(cudaMemset(d_counts_, 0, 2 * sizeof(long long)));
     h_ctl_[0] = 1;
@@ -259,7 +258,6 @@ Engine::~Engine() {
     }
     cudaFreeHost(h_pos_);
     cudaFreeHost(h_forces_);
-    cudaFreeHost(h_fnb_);
     cudaFreeHost(h_results_);
     cudaFreeHost(h_matrix_);
     cudaFreeHost(h_params_);
@@ -1301,7 +1299,7 @@ void Engine::alloc_device() {
     a.merge_w = dalloc<long long>(d_allocs_, (size_t)R_);
     a.results = dalloc<double>(d_allocs_, (size_t)R_ * NUM_RES);
     a.matrix = dalloc<double>(d_allocs_, (size_t)R_ * R_);
-    a.beta = reinterpret_cast<double*>(d_params_ + 40);
+    a.beta = reinterpret_cast<double*>(d_params_ + 32);
     CUDA_CHECK(cudaMemset(a.status, 0, sizeof(Status)));
     CUDA_CHECK(cudaHostGetDevicePointer((void**)&a.h_status, h_status_, 0));
     a.h_results = a.h_matrix = nullptr;
@@ -1485,7 +1483,35 @@ bool Engine::check_status_and_grow() {
     return true;
 }
 
-void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos_pinned, bool host_results) {
+// The device address of a page-locked, mapped host buffer (cudaHostAlloc, or
+// cudaHostRegister with mapping), which kernels can write over the host link; null
+// for other memory.
+static double* host_mapped(double* p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (at.type != cudaMemoryTypeHost || at.devicePointer == nullptr) return nullptr;
+    return static_cast<double*>(at.devicePointer);
+}
+
+// Staged host positions are read over the host link by k_prepare itself, each atom once,
+// in place of a copy before the graph: an energy call of one system took 71.5 -> 68 us at
+// 1,500 atoms, 99 -> 95 at 12,000, 256 -> 252 at 46,000 and 1,323 -> 1,319 at 384,000 (the
+// reads hide behind one another, the copy's start-up did not).  A caller's own page-locked
+// buffer is still copied: the copy checks its extent, a kernel would not.
+void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos, bool host_results) {
+    const bool direct = h_pos && h_pos == h_pos_;
+    struct Reset {  // (the next evaluation may be another kind)
+        Engine* e;
+        double* io0;
+        ~Reset() {
+            if (!e) return;
+            e->h_io_[0] = io0;
+            e->h_ctl_[1] &= ~EVAL_HOST_POSITIONS;
+        }
+    } reset{direct ? this : nullptr, h_io_[0]};
     CUDA_CHECK(cudaSetDevice(dev_));
     if (!layout_ready_) {
         build_layout();
@@ -1500,17 +1526,21 @@ void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos_pin
         h_ctl_[0] = (force_build_ || skin_ <= 0.0) ? 1 : 0;
         force_build_ = false;
         cudaStream_t st = user ? user : s_main_;
+        if (direct) {
+            h_io_[0] = host_mapped(h_pos_);
+            h_ctl_[1] |= EVAL_HOST_POSITIONS;
+        }
         upload_params(st);
         Args a = A_;
-        if (profiling_ || h_pos_pinned || host_results) {
+        if (profiling_ || h_pos || host_results) {
             CUDA_CHECK(cudaHostGetDevicePointer((void**)&a.h_results, h_results_, 0));
             CUDA_CHECK(cudaHostGetDevicePointer((void**)&a.h_matrix, h_matrix_, 0));
         }
         if (d_pos && d_pos != h_io_[0])  // (positions the graph reads in place need no copy)
             CUDA_CHECK(cudaMemcpyAsync((void*)A_.pos_in, d_pos, sizeof(double) * 3 * (size_t)n_in_,
                                        cudaMemcpyDeviceToDevice, st));
-        if (h_pos_pinned)
-            CUDA_CHECK(cudaMemcpyAsync((void*)A_.pos_in, h_pos_pinned, sizeof(double) * 3 * (size_t)n_in_,
+        if (h_pos && !direct)
+            CUDA_CHECK(cudaMemcpyAsync((void*)A_.pos_in, h_pos, sizeof(double) * 3 * (size_t)n_in_,
                                        cudaMemcpyHostToDevice, st));
         if (profiling_) {
             // eager launches bracketed by events, one stream, for per-kernel timings
@@ -1573,8 +1603,8 @@ void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos_pin
     throw Error(6, "Tile list capacity could not be established");
 }
 
-// Page-locked host memory (cudaHostAlloc / cudaHostRegister) can be the source or
-// target of an asynchronous copy without a staging copy.
+// Page-locked host memory (cudaHostAlloc / cudaHostRegister) can be the source of an
+// asynchronous copy without a staging copy.
 static bool is_pinned(const void* p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -1582,19 +1612,6 @@ static bool is_pinned(const void* p) {
         return false;
     }
     return at.type == cudaMemoryTypeHost;
-}
-
-// The device address of a page-locked, mapped host buffer (cudaHostAlloc, or
-// cudaHostRegister with mapping), which kernels can write over the host link; null
-// for other memory.
-static double* host_mapped(double* p) {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (at.type != cudaMemoryTypeHost || at.devicePointer == nullptr) return nullptr;
-    return static_cast<double*>(at.devicePointer);
 }
 
 // Host copy split over a few threads (a single core moves ~10-20 GB/s).
@@ -1614,38 +1631,68 @@ static void par_memcpy(void* dst, const void* src, size_t bytes) {
     for (auto& x : th) x.join();
 }
 
-void Engine::evaluate(double* energies, double* forces, double* forces_nb, double* results, double* matrix) {
-    evaluate_host(nullptr, energies, forces, forces_nb, results, matrix);
-}
-
-void Engine::evaluate_host(const double* pos, double* energies, double* forces, double* forces_nb, double* results,
-                           double* matrix) {
+void Engine::evaluate_host(const double* pos, double* energies, double* forces, double* results, double* matrix) {
     CUDA_CHECK(cudaSetDevice(dev_));
     settle_params();
     const size_t bytes = sizeof(double) * 3 * (size_t)n_in_;
     const bool pin_in = pos && is_pinned(pos);
     // the layout and the profiling path read the staging copy
     if (pos && (!pin_in || !layout_ready_ || profiling_)) par_memcpy(h_pos_, pos, bytes);
-    // positions straight from a pinned caller buffer, else from the pinned staging
-    // copy; forces written by the output kernel over the host link, straight into a
-    // page-locked caller buffer or else into the pinned staging copies
+    // positions copied from a page-locked caller buffer, else taken from the staging copy;
+    // forces written by the output kernel over the host link, straight into a
+    // page-locked caller buffer or else into the staging copy
     double* const zc = forces ? host_mapped(forces) : nullptr;
     h_io_[1] = zc ? zc : (forces ? host_mapped(h_forces_) : nullptr);
-    h_io_[3] = forces_nb ? host_mapped(h_fnb_) : nullptr;
     try {
         run(s_main_, nullptr, pin_in && !profiling_ ? pos : h_pos_);
     } catch (...) {
-        h_io_[1] = h_io_[3] = nullptr;
+        h_io_[1] = nullptr;
         throw;
     }
-    h_io_[1] = h_io_[3] = nullptr;  // (the graph that read them has finished)
+    h_io_[1] = nullptr;  // (the graph that read it has finished)
     if (forces && !zc) par_memcpy(forces, h_forces_, bytes);
-    if (forces_nb) par_memcpy(forces_nb, h_fnb_, bytes);
     for (int r = 0; r < R_; r++) {
         if (energies) energies[r] = h_results_[(size_t)r * NUM_RES + RES_ENERGY];
     }
     if (results) std::memcpy(results, h_results_, sizeof(double) * NUM_RES * (size_t)R_);
     if (matrix) std::memcpy(matrix, h_matrix_, sizeof(double) * (size_t)R_ * R_);
+}
+
+static int output_mode(bool merged, bool state1) {
+    return (state1 ? EVAL_ADD_STATE1 : 0) | (merged ? 0 : EVAL_NO_MERGED);
+}
+
+const double* Engine::evaluate_forces(bool merged, bool state1, double* results) {
+    CUDA_CHECK(cudaSetDevice(dev_));
+    settle_params();
+    h_io_[1] = host_mapped(h_forces_);
+    h_ctl_[1] = output_mode(merged, state1);
+    try {
+        run(s_main_, nullptr, h_pos_);
+    } catch (...) {
+        h_io_[1] = nullptr;
+        h_ctl_[1] = 0;
+        throw;
+    }
+    h_io_[1] = nullptr;
+    h_ctl_[1] = 0;
+    std::memcpy(results, h_results_, sizeof(double) * NUM_RES * (size_t)R_);
+    return h_forces_;
+}
+
+const double* Engine::output_forces(bool merged, bool state1) {
+    CUDA_CHECK(cudaSetDevice(dev_));
+    settle_params();
+    h_io_[1] = host_mapped(h_forces_);
+    h_ctl_[1] = output_mode(merged, state1);
+    upload_params(s_main_);
+    launch_output(A_, s_main_);
+    CUDA_CHECK(cudaGetLastError());
+    CUDA_CHECK(cudaStreamSynchronize(s_main_));
+    params_pending_ = false;
+    h_io_[1] = nullptr;  // (the transfer that read them has finished)
+    h_ctl_[1] = 0;
+    return h_forces_;
 }
 
 void Engine::run_device(const double* d_pos, cudaStream_t stream) {

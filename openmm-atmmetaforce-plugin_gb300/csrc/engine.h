@@ -83,12 +83,15 @@ public:
     // evaluations run and how many of them built the lists (synchronises the device)
     void list_counts(long long* evals, long long* builds) const;
 
-    // Host path: positions from the staging copy; outputs to host (nullable).
-    void evaluate(double* energies, double* forces, double* forces_nb, double* results, double* matrix);
-    // Host path with the caller's positions (nullable: the staging copy).  Page-locked
-    // caller buffers are copied from / to directly; others go through pinned staging.
-    void evaluate_host(const double* pos, double* energies, double* forces, double* forces_nb, double* results,
-                       double* matrix);
+    // Host path with the caller's positions (nullable: the staging copy); outputs to host
+    // (nullable).  Page-locked caller buffers are copied from and written directly; others
+    // go through pinned staging.
+    void evaluate_host(const double* pos, double* energies, double* forces, double* results, double* matrix);
+    // Host path from the staged positions: the sum of the merged ATM forces and the
+    // state-1 nonbonded forces, as asked for, formed on the device; valid until the next call.
+    const double* evaluate_forces(bool merged, bool state1, double* results);
+    // The same of the last evaluation, without another one.
+    const double* output_forces(bool merged, bool state1);
     // Device path on the caller's stream.
     void evaluate_device(const double* d_pos, double* d_forces, double* d_results, cudaStream_t stream);
     // Device path without output copies: after it returns, forces_device() and
@@ -182,9 +185,9 @@ private:
     void fetch_nonbonded_params();
     void refresh_param_tables();
     void settle_params();
-    // host_results (implied by h_pos_pinned): the result records and the matrix also end
-    // in h_results_ / h_matrix_
-    void run(cudaStream_t user, const double* d_pos, const double* h_pos_pinned = nullptr, bool host_results = false);
+    // h_pos: positions from page-locked host memory.  host_results (implied by h_pos): the
+    // result records and the matrix also end in h_results_ / h_matrix_
+    void run(cudaStream_t user, const double* d_pos, const double* h_pos = nullptr, bool host_results = false);
     bool check_status_and_grow();
     void destroy_graphs();
 
@@ -269,7 +272,6 @@ private:
     // pinned host staging
     double* h_pos_ = nullptr;      // 3*n_in
     double* h_forces_ = nullptr;   // 3*n_in
-    double* h_fnb_ = nullptr;      // 3*n_in
     double* h_results_ = nullptr;  // R*NUM_RES
     double* h_matrix_ = nullptr;   // R*R
     // The per-evaluation parameters in one page-locked block (list control word,
@@ -285,9 +287,9 @@ private:
     bool params_pending_ = false;
     RepDev* h_reps_ = nullptr;     // R
     double* h_beta_ = nullptr;
-    int* h_ctl_ = nullptr;         // list control word
+    int* h_ctl_ = nullptr;         // list control word, EvalMode bits
     double** h_io_ = nullptr;      // caller buffers of the next evaluations (Args::io): positions,
-                                   // forces, result records, state-1 nonbonded forces
+                                   // forces, result records
     Status* h_status_ = nullptr;
 
     // device buffers

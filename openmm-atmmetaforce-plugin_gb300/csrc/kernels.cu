@@ -151,8 +151,15 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
         int o = a.orig[s];
         const int nreal = __popc(__ballot_sync(FULL_MASK, o >= 0));  // padding sits at the end of a block
         if (o < 0) o = a.orig[b * kTile];  // padding copies the block's first atom
-        const double* p = (a.io[0] ? a.io[0] : a.pos_in) + 3 * (size_t)(R.in_off + o);
+        const size_t io = 3 * (size_t)(R.in_off + o);
+        const double* p = (a.io[0] ? a.io[0] : a.pos_in) + io;
         double xd = p[0], yd = p[1], zd = p[2];
+        if ((a.list_ctl[1] & EVAL_HOST_POSITIONS) && a.orig[s] >= 0) {  // (the exceptions read them again)
+            double* to = const_cast<double*>(a.pos_in) + io;
+            to[0] = xd;
+            to[1] = yd;
+            to[2] = zd;
+        }
         float x = (float)xd, y = (float)yd, z = (float)zd;
         // a position whose reduced coordinates lie safely inside (0, 1) (by 1e-5, far
         // beyond the FP32 estimate's error) is in the unit cell already: the FP64 wrap
@@ -338,7 +345,7 @@ __device__ __forceinline__ void exceptions_cta(const Args& a, int c) {
         int4 ij = a.exc_ij[e];
         ExcParam p = a.exc_p[e];
         const RepDev& R = a.reps[ij.z];
-        const double* pos = a.io[0] ? a.io[0] : a.pos_in;
+        const double* pos = a.io[0] && !(a.list_ctl[1] & EVAL_HOST_POSITIONS) ? a.io[0] : a.pos_in;
         const double* xi = pos + 3 * (size_t)ij.x;
         const double* xj = pos + 3 * (size_t)ij.y;
         int si = a.slot_of[ij.x], sj = a.slot_of[ij.y];
@@ -1358,7 +1365,9 @@ void launch_finalize(const Args& a, cudaStream_t s) {
 // slot_of), so that a warp's 32 atoms are 768 contiguous bytes of the output,
 // written as 16-byte words through shared memory.  The output is f_out, or a
 // page-locked host buffer the caller passed (io[1]), written over the host link
-// without a separate copy.
+// without a separate copy.  The sum over force groups that a single system's state asks
+// for is formed here too (EvalMode): written apart and added on the host, the two force
+// arrays cost a 23,558-atom system 280 us a state against 215.
 constexpr int kOutThreads = 256;
 
 // Entry idx of the replicas x states energy matrix, beta * (e0(r; dir_s) + W_s(usc_s(u(r;
@@ -1413,8 +1422,8 @@ __global__ void __launch_bounds__(kOutThreads) k_output(Args a, int nmat) {
     }
     const int g = (blockIdx.x - nmat) * kOutThreads + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double* const fo = a.io[1] ? a.io[1] : a.f_out;
-    double* const fnb = a.io[3];
-    double f[3] = {0.0, 0.0, 0.0}, fb[3] = {0.0, 0.0, 0.0};
+    const int mode = a.list_ctl[1];
+    double f[3] = {0.0, 0.0, 0.0};
     if (g < a.n_in) {
         const int s = a.slot_of[g];
         const int rep = a.block_rep[s >> 5];
@@ -1426,15 +1435,14 @@ __global__ void __launch_bounds__(kOutThreads) k_output(Args a, int nmat) {
         for (int k = 0; k < 3; k++) {
             const long long f1 = (long long)a.F[(size_t)k * a.NA + s];
             const long long v = merged_fix(f1, (long long)a.F[(size_t)(3 + k) * a.NA + s], a.full, w32);
-            f[k] = R.var_nb ? fix_scaled(v) : 0.0;
-            if (fnb) fb[k] = fix_scaled(f1);
+            f[k] = R.var_nb && !(mode & EVAL_NO_MERGED) ? fix_scaled(v) : 0.0;
+            if (mode & EVAL_ADD_STATE1) f[k] += fix_scaled(f1);
         }
     }
     const int g0 = g - lane;  // the warp's first atom
     const int nv = min(32, a.n_in - g0);
     if (nv <= 0) return;
     store_forces(fo + 3 * (size_t)g0, f, s_f[w], lane, nv);
-    if (fnb) store_forces(fnb + 3 * (size_t)g0, fb, s_f[w], lane, nv);
 }
 
 void launch_output(const Args& a, cudaStream_t s) {

@@ -73,6 +73,14 @@ __host__ __device__ inline int spread_row_stride(int n) {
     return n;
 }
 
+// How an evaluation takes its positions and what its forces are (a control word, so that
+// one recorded graph serves every mode).
+enum EvalMode {
+    EVAL_HOST_POSITIONS = 1,  // io[0] is the engine's page-locked staging copy: read once, into pos_in
+    EVAL_ADD_STATE1 = 2,      // the state-1 nonbonded forces are added to the output
+    EVAL_NO_MERGED = 4        // the merged ATM forces are left out of it
+};
+
 // Row kinds of the pair-tile lists.
 enum RowKind { ROW_STATE1 = 0, ROW_STATE2 = 1, ROW_DIFF1 = 2, ROW_DIFF2 = 3 };
 
@@ -225,7 +233,7 @@ struct Args {
     float rcl2;               // (rc + skin)^2
     float skin_half2;         // (skin / 2)^2
     float4* posq_ref;         // NA: positions at the last build
-    const int* list_ctl;      // device control word: [0] = 1 forces a build
+    const int* list_ctl;      // device control words: [0] = 1 forces a build, [1]: EvalMode bits
     unsigned* rep_hmax;       // R: largest half-extent norm of a block (float bits; triclinic boxes)
     int any_tric;             // 1: some replica's box is triclinic
     long long* list_counts;   // device: evaluations, list builds
@@ -241,8 +249,7 @@ struct Args {
                               // caller's device positions, read in place of pos_in; io[1] the
                               // caller's force buffer (device, or page-locked host memory
                               // written over the host link) in place of f_out; io[2] the
-                              // caller's device result records (a copy of results); io[3] the
-                              // state-1 nonbonded force (3*n_in); null: unused
+                              // caller's device result records (a copy of results); null: unused
     // slot arrays
     const int* orig;          // NA: user index within the replica, -1 for padding
     float* qs;                // NA: charge * sqrt(1/(4 pi eps0))
