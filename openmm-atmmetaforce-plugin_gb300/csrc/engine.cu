@@ -1412,14 +1412,22 @@ void Engine::record(cudaStream_t st, const Args& a, bool output) {
         launch_gather(a, ps);
         if (tune_pme_stream_) CUDA_CHECK(cudaEventRecord(ev_join_, s_pme_));
     }
+    // without PME the exceptions are the second stream's, beside the list building and
+    // the tiles (2,394 atoms, us a state: 78 with their 4 us kernel after the tiles, 74)
+    const bool exc_beside = !pme && a.exc_ctas > 0;
+    if (exc_beside) {
+        CUDA_CHECK(cudaEventRecord(ev_fork_, st));
+        CUDA_CHECK(cudaStreamWaitEvent(s_pme_, ev_fork_, 0));
+        launch_exceptions(a, s_pme_);
+        CUDA_CHECK(cudaEventRecord(ev_join_, s_pme_));
+    }
     if (a.fused) {
         launch_find_tiles(a, st);
     } else {
         launch_find(a, st);
         launch_tiles(a, tile_launch_grid(), st);
     }
-    if (!pme) launch_exceptions(a, st);
-    if (pme && tune_pme_stream_) CUDA_CHECK(cudaStreamWaitEvent(st, ev_join_, 0));
+    if ((pme && tune_pme_stream_) || exc_beside) CUDA_CHECK(cudaStreamWaitEvent(st, ev_join_, 0));
     launch_finalize(a, st);
     if (output) launch_output(a, st);
 }
