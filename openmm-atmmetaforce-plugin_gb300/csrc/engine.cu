@@ -636,7 +636,11 @@ static void parallel_for(int n, const F& f) {
             }
     };
     std::vector<std::thread> th;
-    for (int t = 1; t < nt; t++) th.emplace_back(work);
+    try {
+        th.reserve(nt - 1);
+        for (int t = 1; t < nt; t++) th.emplace_back(work);
+    } catch (...) {  // no thread to be had: those started and this one do the work
+    }
     work();
     for (auto& t : th) t.join();
     if (err) std::rethrow_exception(err);

@@ -5,10 +5,12 @@
 //              block bounding boxes; zero the force accumulators and charge grids;
 //              decide whether the lists are built
 //   find     : one warp per tile row -> compacted list of interacting tiles
-//   tiles    : persistent warps over the tile list: LJ + reaction field / Ewald
-//              direct space, tile rotation by warp shuffles, fixed-point forces
+//   tiles    : warps over the tile list (persistent ones when it is large): LJ +
+//              reaction field / Ewald direct space, tile rotation by warp shuffles,
+//              fixed-point forces
 //   spread / transforms with the convolution / gather : smooth PME; the exceptions
-//              (FP64 and FP32) and Ewald exclusion corrections beside the spreading
+//              (FP64 and FP32) and Ewald exclusion corrections beside the spreading,
+//              or without PME beside find and tiles
 //   finalize : FP64 energies, soft-core + softplus merge (ATM scalars)
 //   output   : hybrid forces F1 + s' (F2 - F1) in user order, and the replicas x
 //              states reduced-energy matrix

@@ -230,7 +230,7 @@ __device__ __forceinline__ void stage_r(const float2* src, float2* dst, const Ff
 // sequence, so the twiddles are broadcast reads.  The stage was bound by those
 // remainders' integer instructions: with one output per item and `%` per term,
 // 8 replicas of a 68^3 grid (4 x 17) took 208 / 216 / 201 us in the three kernels,
-// the rest of each about 25 us.
+// the rest of each about 25 us; now 84 / 87 / 76.
 constexpr int kGenOut = 4;
 
 template <bool INV>
