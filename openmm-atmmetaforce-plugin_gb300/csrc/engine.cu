@@ -830,6 +830,7 @@ void Engine::build_layout() {
     groups_.clear();
     fft_tw_.clear();
     fft_stages_.clear();
+    fft_roots_.clear();
     fft_plane_.clear();
     fft_conv_.clear();
     use_fft_ = false;
@@ -876,7 +877,7 @@ void Engine::build_layout() {
                         const double ph = -2.0 * kPi * k / rd.K[a];
                         fft_tw_.push_back(make_float2((float)std::cos(ph), (float)std::sin(ph)));
                     }
-                    t[2] = fft_plan_stages(rd.K[a], fft_stages_);
+                    t[2] = fft_plan_stages(rd.K[a], fft_stages_, fft_tw_.data() + t[1], fft_roots_);
                     it = tables.emplace(rd.K[a], t).first;
                 }
                 rd.mod_off[a] = it->second[0];
@@ -1264,6 +1265,7 @@ void Engine::alloc_device() {
         a.use_fft = use_fft_ ? 1 : 0;
         a.fft_tw = dupload(d_allocs_, fft_tw_);
         a.fft_stages = dupload(d_allocs_, fft_stages_);
+        a.fft_roots = fft_roots_.empty() ? nullptr : reinterpret_cast<float4*>(dupload(d_allocs_, fft_roots_));
         a.fft_plane_ctas = (int)fft_plane_.size();
         a.fft_plane = dupload(d_allocs_, fft_plane_);
         a.fft_plane_smem = fft_plane_smem_;

@@ -263,6 +263,7 @@ private:
     bool use_fft_ = false;
     std::vector<float2> fft_tw_;
     std::vector<FftStage> fft_stages_;
+    std::vector<float2> fft_roots_;
     std::vector<int2> fft_plane_;
     std::vector<int4> fft_conv_;
     int fft_plane_smem_ = 0, fft_conv_smem_ = 0;

@@ -97,7 +97,8 @@ enum Res {
 struct FftStage {
     int R, Ns, nb, step;
     unsigned mNs;
-    int pad[3];
+    int tab;  // prime stages: their roots in fft_roots (16-byte words)
+    int pad[2];
 };
 
 struct RepDev {
@@ -329,6 +330,7 @@ struct Args {
     int use_fft;              // 1: k_fft_zy / k_fft_x_conv / k_ifft_yz
     const float2* fft_tw;     // twiddles w_N^k = exp(-2 pi i k / N), per replica and dimension
     const FftStage* fft_stages;  // stage plans (RepDev::fft_plan indexes them)
+    const float4* fft_roots;     // roots of the prime stages, two per word, in reading order
     int fft_plane_ctas;       // (grid, x-plane) CTAs of all replicas
     const int2* fft_plane;    //   (replica, grid * K0 + x)
     int fft_plane_smem;       // dynamic shared memory of a plane CTA (bytes)
@@ -363,8 +365,9 @@ void launch_fft_forward(const Args& a, cudaStream_t s);
 void launch_fft_conv(const Args& a, cudaStream_t s);
 void launch_fft_inverse(const Args& a, cudaStream_t s);
 int fft_plane_smem_bytes(int K1, int K2);
-// Stages of a 1D transform of length N appended to out; returns first | count << 24.
-int fft_plan_stages(int N, std::vector<FftStage>& out);
+// Stages of a 1D transform of length N (twiddles tw) appended to out, the roots of its prime
+// stages to roots; returns first | count << 24.
+int fft_plan_stages(int N, std::vector<FftStage>& out, const float2* tw, std::vector<float2>& roots);
 void launch_influence(float* G, const float* moduli, const int* mod_off, const int* K, const double* recip,
                       double volume, double alpha, cudaStream_t s);
 int fft_conv_smem_bytes(int K0, int nz);

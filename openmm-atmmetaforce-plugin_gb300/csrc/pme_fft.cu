@@ -223,42 +223,44 @@ __device__ __forceinline__ void stage_r(const float2* src, float2* dst, const Ff
 
 // Direct DFT stage for a prime factor R outside the dedicated radices.  A work item
 // is kGenOut outputs m of one butterfly: each input is read from shared memory once
-// for all of them, and the exponent of the combined twiddle and DFT root,
-// w_N^{r k step} w_R^{r m} = w_N^{r (k step + m nb)} (R nb = N), advances by a
-// constant below N per input, one conditional subtraction in place of two runtime
-// remainders.  Neighbouring threads share (butterfly, outputs) and differ in the
-// sequence, so the twiddles are broadcast reads.  The stage was bound by those
-// remainders' integer instructions: with one output per item and `%` per term,
-// 8 replicas of a 68^3 grid (4 x 17) took 208 / 216 / 201 us in the three kernels,
-// the rest of each about 25 us; now 84 / 87 / 76.
-constexpr int kGenOut = 4;
+// for all of them.  The combined twiddle and DFT root of input r, w_N^{r k step} w_R^{r m}
+// = w_N^{r (k step + m nb)} (R nb = N), comes from a table in the order of the reads,
+// [k][m / kGenOut][r][m % kGenOut] (fft_plan_stages; the values of the twiddle table):
+// neighbouring threads share (butterfly, outputs) and differ in the sequence, so these are
+// 16-byte broadcast loads of two roots.  The stage was bound by the instructions that find
+// the roots: 8 replicas of a 68^3 grid (4 x 17) took 208 / 216 / 201 us in the three
+// kernels with one output per item and a remainder per term, 84 / 87 / 76 with four outputs
+// and the exponents advanced by additions, and 75 / 75 / 58 from the table with six (the
+// first beside the finder; the rest of each about 25 us).  Outputs per item 4 / 6 / 8, us a
+// pass: these 1,090 / 1,072 / 1,095, three sizes of box with 45, 34 and 46 points 381 / 370
+// / 383 (six leave one output of 17 and 23 over); packed FP32 instructions no faster.
+constexpr int kGenOut = 6;
 
 template <bool INV>
-__device__ __forceinline__ void stage_generic(const float2* src, float2* dst, const FftStage& p, int N,
-                                              const FastDiv& fq, int ss, int es, const float2* tw) {
-    const int R = p.R, nb = p.nb, Ns = p.Ns, step = p.step;
-    const int items = nb * ((R + kGenOut - 1) / kGenOut) * (int)fq.d;
+__device__ __forceinline__ void stage_generic(const float2* src, float2* dst, const FftStage& p, const FastDiv& fq,
+                                              int ss, int es, const float4* roots) {
+    const int R = p.R, nb = p.nb, Ns = p.Ns, ng = (R + kGenOut - 1) / kGenOut;
+    const int items = nb * ng * (int)fq.d;
     const FastDiv fnb(nb), fns((unsigned)Ns, p.mNs);
+    const int sr = nb * es;
     for (int w = threadIdx.x; w < items; w += blockDim.x) {
         const int t = (int)fq.div((unsigned)w), q = w - t * (int)fq.d;  // t: (outputs m0 .., butterfly j)
         const int mg = (int)fnb.div((unsigned)t), j = t - mg * nb, m0 = mg * kGenOut;
         const int jn = (int)fns.div((unsigned)j), k = j - jn * Ns;
         const float2* s = src + q * ss + j * es;
+        const float4* root = roots + p.tab + (k * ng + mg) * R * (kGenOut / 2);
         float2 acc[kGenOut];
-        int e[kGenOut], inc[kGenOut];
 #pragma unroll
-        for (int u = 0; u < kGenOut; u++) {
-            acc[u] = make_float2(0.f, 0.f);
-            e[u] = 0;
-            inc[u] = m0 + u < R ? k * step + (m0 + u) * nb : 0;
-        }
+        for (int u = 0; u < kGenOut; u++) acc[u] = make_float2(0.f, 0.f);
+#pragma unroll 1
         for (int r = 0; r < R; r++) {
-            const float2 x = s[r * nb * es];
+            const float2 x = *s;
+            s += sr;
 #pragma unroll
-            for (int u = 0; u < kGenOut; u++) {
-                acc[u] = cadd(acc[u], cmul(x, twid<INV>(tw, e[u])));
-                e[u] += inc[u];
-                e[u] -= e[u] >= N ? N : 0;
+            for (int u = 0; u < kGenOut; u += 2) {
+                const float4 v = __ldg(root++);
+                acc[u] = cadd(acc[u], cmul(x, make_float2(v.x, INV ? -v.y : v.y)));
+                acc[u + 1] = cadd(acc[u + 1], cmul(x, make_float2(v.z, INV ? -v.w : v.w)));
             }
         }
         float2* d = dst + q * ss + (jn * Ns * R + k) * es;
@@ -290,7 +292,7 @@ __device__ int fft_seqs(const Args& a, int plan, float2* buf0, float2* buf1, int
                 case 3: stage_r<3, INV, false>(src, dst, p, fq, ss, es, tw); break;
                 case 5: stage_r<5, INV, false>(src, dst, p, fq, ss, es, tw); break;
                 case 7: stage_r<7, INV, false>(src, dst, p, fq, ss, es, tw); break;
-                default: stage_generic<INV>(src, dst, p, N, fq, ss, es, tw); break;
+                default: stage_generic<INV>(src, dst, p, fq, ss, es, a.fft_roots); break;
             }
         } else {
             switch (p.R) {
@@ -300,7 +302,7 @@ __device__ int fft_seqs(const Args& a, int plan, float2* buf0, float2* buf1, int
                 case 3: stage_r<3, INV, true>(src, dst, p, fq, ss, es, tw); break;
                 case 5: stage_r<5, INV, true>(src, dst, p, fq, ss, es, tw); break;
                 case 7: stage_r<7, INV, true>(src, dst, p, fq, ss, es, tw); break;
-                default: stage_generic<INV>(src, dst, p, N, fq, ss, es, tw); break;
+                default: stage_generic<INV>(src, dst, p, fq, ss, es, a.fft_roots); break;
             }
         }
         __syncthreads();
@@ -573,7 +575,7 @@ int fft_plane_smem_bytes(int K1, int K2) {
 
 // Radices 8 (as many as divide N), then 4 or 2 for the rest of the power of two,
 // then 3, 5, 7 and any other prime factor, smallest first.
-int fft_plan_stages(int N, std::vector<FftStage>& out) {
+int fft_plan_stages(int N, std::vector<FftStage>& out, const float2* tw, std::vector<float2>& roots) {
     std::vector<int> rad;
     int n = N;
     while (n % 8 == 0) { rad.push_back(8); n /= 8; }
@@ -590,6 +592,14 @@ int fft_plan_stages(int N, std::vector<FftStage>& out) {
         st.nb = N / R;
         st.step = N / (Ns * R);
         st.mNs = Ns > 1 ? (unsigned)((0x100000000ull + (unsigned long long)Ns - 1) / (unsigned long long)Ns) : 0u;
+        if (R > 8) {  // stage_generic's roots; outputs past R are not stored
+            st.tab = (int)(roots.size() / 2);
+            for (int k = 0; k < Ns; k++)
+                for (int m0 = 0; m0 < R; m0 += kGenOut)
+                    for (int r = 0; r < R; r++)
+                        for (int m = m0; m < m0 + kGenOut; m++)
+                            roots.push_back(m < R ? tw[(long long)r * (k * st.step + m * st.nb) % N] : make_float2(0.f, 0.f));
+        }
         out.push_back(st);
         Ns *= R;
     }

@@ -35,10 +35,16 @@ def test_grids_of_odd_and_multiple_of_four_sizes_in_one_batch(diff):
 
 @pytest.mark.parametrize("diff", [0, 1], ids=["two-states", "difference"])
 def test_grids_with_prime_factors_beyond_the_dedicated_radices(diff):
-    """The direct DFT stage: primes 11 to 37, one to three past a multiple of its
+    """The direct DFT stage: primes 11 to 37, one or five past a multiple of its
     outputs per work item, alone (23, 29, 31, 37) and after other stages (22, 26,
     33, 34, 38, 39)."""
     _check([(22, 23, 26), (31, 29, 37), (34, 39, 38), (33, 22, 22), (26, 22, 34)], diff)
+
+
+@pytest.mark.parametrize("grid", [(121, 24, 22), (24, 121, 26), (22, 26, 121), (101, 23, 24), (143, 20, 21)])
+def test_grids_with_two_prime_stages_or_a_long_one(grid):
+    """Roots of a prime stage after another one (121, 143), and of one prime (101)."""
+    _check([grid], 1)
 
 
 @pytest.mark.parametrize("ligand", [7, 8, 9, 33], ids=lambda n: f"ligand{n}")
