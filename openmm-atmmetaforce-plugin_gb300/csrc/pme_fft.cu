@@ -34,7 +34,17 @@
 
 namespace atm {
 
+// Threads of a CTA of the three kernels: kFftThreads, or twice as many (kWide) where the
+// time is a CTA's own chain of loops: planes of at least kWideMin points and at most two
+// per SM (x slabs, whose CTA holds two planes: one).  us of 20 MD steps, 256 / 512 threads:
+// 1 x 23,558 atoms (112 planes of 56 x 29 points) 2,936 / 2,808, 2 x 23,558 3,896 / 3,787,
+// 1 x 46,001 (69 points) 4,930 / 4,127, 2 x 46,001 7,240 / 6,742; a state of one 46,001-atom
+// system 414 / 386.  Smaller or more planes lose: 4 x 5,000 (288 of 36 x 19) 3,304 / 3,500,
+// 3 x 12,000 (270 of 45 x 23) 3,331 / 3,437, 4 x 8,009 (352) 240 / 249 a pass, 22 x 23,558
+// 973 / 1,036.
 constexpr int kFftThreads = 256;
+constexpr int kWide = 2 * kFftThreads;
+constexpr int kWideMin = 1500;
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -325,7 +335,8 @@ __device__ __forceinline__ void load_tw(const Args& a, const RepDev& R, int d, f
 // ceil(K1/2) x K2 and K1 x (K2/2 + 1) complex values, and the y and z twiddles.
 // The spectrum of a grid is laid out [ky][x][kz] (kz < K2/2 + 1), so that the x
 // transforms of one ky read one contiguous slab.
-__global__ void __launch_bounds__(kFftThreads, 5) k_fft_zy(Args a) {
+template <int T>
+__global__ void __launch_bounds__(T, T == kWide ? 2 : 5) k_fft_zy(Args a) {
     extern __shared__ float2 sh[];
     const int2 pc = a.fft_plane[blockIdx.x];  // (replica, grid * K0 + x)
     const RepDev& R = a.reps[pc.x];
@@ -389,7 +400,8 @@ __global__ void __launch_bounds__(kFftThreads, 5) k_fft_zy(Args a) {
     }
 }
 
-__global__ void __launch_bounds__(kFftThreads, 5) k_ifft_yz(Args a) {
+template <int T>
+__global__ void __launch_bounds__(T, T == kWide ? 2 : 5) k_ifft_yz(Args a) {
     extern __shared__ float2 sh[];
     const int2 pc = a.fft_plane[blockIdx.x];
     const RepDev& R = a.reps[pc.x];
@@ -458,7 +470,8 @@ __global__ void __launch_bounds__(kFftThreads, 5) k_ifft_yz(Args a) {
 
 // x transforms and the convolution of one (replica, ky, [kz0, kz1)) slab of both
 // grids.  Shared layout: M[x][c], c < 2 nz (grid 0's columns, then grid 1's).
-__global__ void __launch_bounds__(kFftThreads, 4) k_fft_x_conv(Args a) {
+template <int T>
+__global__ void __launch_bounds__(T, T == kWide ? 2 : 4) k_fft_x_conv(Args a) {
     extern __shared__ float2 sh[];
     __shared__ double red[2][kFftThreads / 32];
     const int4 cc = a.fft_conv[blockIdx.x];  // (replica, ky, kz0, kz1)
@@ -492,8 +505,9 @@ __global__ void __launch_bounds__(kFftThreads, 4) k_fft_x_conv(Args a) {
     // B-spline moduli; the half spectrum counts kz in (0, K2/2) twice.  Each
     // thread's terms are summed exactly to about 2^-48 (TwoSum), then in FP64.
     float sa = 0.f, ca = 0.f, sb = 0.f, cb = 0.f;
+    // (by the first kFftThreads threads: the sums are the same at either width)
 #pragma unroll 2
-    for (int w = threadIdx.x; w < K0 * nz; w += blockDim.x) {
+    for (int w = threadIdx.x < kFftThreads ? threadIdx.x : K0 * nz; w < K0 * nz; w += kFftThreads) {
         const int x = (int)fn.div((unsigned)w), c = w - x * nz, kz = kz0 + c;
         const float G = gsh[w];
         const float wgt = (kz == 0 || 2 * kz == K2) ? 1.0f : 2.0f;
@@ -510,7 +524,7 @@ __global__ void __launch_bounds__(kFftThreads, 4) k_fft_x_conv(Args a) {
         ea += __shfl_xor_sync(0xffffffffu, ea, o);
         eb += __shfl_xor_sync(0xffffffffu, eb, o);
     }
-    if ((threadIdx.x & 31) == 0) {
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < kFftThreads) {
         red[0][threadIdx.x >> 5] = ea;
         red[1][threadIdx.x >> 5] = eb;
     }
@@ -610,22 +624,45 @@ int fft_conv_smem_bytes(int K0, int nz) {
     return (int)sizeof(float2) * (2 * K0 * 2 * nz + K0) + (int)sizeof(float) * ((K0 * nz + 1) & ~1);
 }
 
+// points: of the largest plane, from its buffers' bytes
+static bool fft_wide(int planes, int points) {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return planes <= 2 * sms && points >= kWideMin;
+}
+
+template <typename K>
+static void launch_fft(K kernel, int threads, int ctas, int smem, const Args& a, cudaStream_t s) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    kernel<<<ctas, threads, smem, s>>>(a);
+}
+
 void launch_fft_forward(const Args& a, cudaStream_t s) {
     if (a.fft_plane_ctas <= 0) return;
-    cudaFuncSetAttribute(k_fft_zy, cudaFuncAttributeMaxDynamicSharedMemorySize, a.fft_plane_smem);
-    k_fft_zy<<<a.fft_plane_ctas, kFftThreads, a.fft_plane_smem, s>>>(a);
+    if (fft_wide(a.fft_plane_ctas, a.fft_plane_smem / 16))
+        launch_fft(k_fft_zy<kWide>, kWide, a.fft_plane_ctas, a.fft_plane_smem, a, s);
+    else
+        launch_fft(k_fft_zy<kFftThreads>, kFftThreads, a.fft_plane_ctas, a.fft_plane_smem, a, s);
 }
 
 void launch_fft_conv(const Args& a, cudaStream_t s) {
     if (a.conv_ctas <= 0) return;
-    cudaFuncSetAttribute(k_fft_x_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, a.fft_conv_smem);
-    k_fft_x_conv<<<a.conv_ctas, kFftThreads, a.fft_conv_smem, s>>>(a);
+    if (fft_wide(2 * a.conv_ctas, a.fft_conv_smem / 36))
+        launch_fft(k_fft_x_conv<kWide>, kWide, a.conv_ctas, a.fft_conv_smem, a, s);
+    else
+        launch_fft(k_fft_x_conv<kFftThreads>, kFftThreads, a.conv_ctas, a.fft_conv_smem, a, s);
 }
 
 void launch_fft_inverse(const Args& a, cudaStream_t s) {
     if (a.fft_plane_ctas <= 0) return;
-    cudaFuncSetAttribute(k_ifft_yz, cudaFuncAttributeMaxDynamicSharedMemorySize, a.fft_plane_smem);
-    k_ifft_yz<<<a.fft_plane_ctas, kFftThreads, a.fft_plane_smem, s>>>(a);
+    if (fft_wide(a.fft_plane_ctas, a.fft_plane_smem / 16))
+        launch_fft(k_ifft_yz<kWide>, kWide, a.fft_plane_ctas, a.fft_plane_smem, a, s);
+    else
+        launch_fft(k_ifft_yz<kFftThreads>, kFftThreads, a.fft_plane_ctas, a.fft_plane_smem, a, s);
 }
 
 }  // namespace atm
