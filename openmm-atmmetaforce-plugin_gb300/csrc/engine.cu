@@ -1178,6 +1178,11 @@ void Engine::alloc_device() {
         a.displ_in = dupload(d_allocs_, d);
     }
     a.slot_of = dupload(d_allocs_, slot_of_);
+    {
+        std::vector<int> first(in_off_);
+        first.push_back(n_in_);
+        a.in_first = dupload(d_allocs_, first);
+    }
     a.f_out = dalloc<double>(d_allocs_, 3 * (size_t)n_in_);
     a.io = reinterpret_cast<double**>(d_params_ + 8);
     a.orig = dupload(d_allocs_, orig_);

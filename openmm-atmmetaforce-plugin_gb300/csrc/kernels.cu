@@ -1536,10 +1536,11 @@ __global__ void __launch_bounds__(kInThreads) k_update_inputs(Args a, DeviceInpu
         a.exc_p[e].w = in.ke * in.q[ij.x] * in.q[ij.y];
     } else {
         __shared__ double red[kInThreads / 32];
-        const RepDev& R = a.reps[b - natom - nexc];
+        // (the replica table would do, but new buffers hold it only from their first evaluation on)
+        const int first = a.in_first[b - natom - nexc], last = a.in_first[b - natom - nexc + 1];
         double t = 0.0;
-        for (int i = threadIdx.x; i < R.n; i += kInThreads) {
-            const double q = in.q[R.in_off + i];
+        for (int i = first + threadIdx.x; i < last; i += kInThreads) {
+            const double q = in.q[i];
             t += q * q;
         }
 #pragma unroll

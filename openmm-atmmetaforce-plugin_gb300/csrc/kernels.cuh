@@ -245,6 +245,7 @@ struct Args {
     const double* pos_in;     // 3*n_in
     const double* displ_in;   // 3*n_in
     const int* slot_of;       // n_in
+    const int* in_first;      // R + 1: each replica's first atom in the caller's arrays, and n_in
     double* f_out;            // 3*n_in (ATM force)
     double* const* io;        // device cells, copied from the host when they change: io[0] the
                               // caller's device positions, read in place of pos_in; io[1] the
