@@ -247,8 +247,8 @@ int atm_batch_set_nonbonded_parameters(atm_batch_t b, int replica, const double*
 /* No counterpart in the reference.  The displacements (sum n x 3), charges, sigmas,
  * epsilons (sum n) and lambda1, lambda2, alpha, u0, w0 (R x 5) of every replica from
  * device memory, as the entry points above set them: compared with the batch's on the
- * device, on the given stream, which the call waits for; only what differs is taken
- * over (on that stream). */
+ * device, on the given stream; only what differs is taken over.  The call waits for the
+ * stream: when it returns, the new values are in force for evaluations on every stream. */
 int atm_batch_set_inputs_device(atm_batch_t b, const double* d_displ, const double* d_charge, const double* d_sigma,
                                 const double* d_epsilon, const double* d_params, void* stream);
 /* No counterpart in the reference (the adjoint of the ATM energy).  Gradients of

@@ -1883,8 +1883,9 @@ void Engine::set_inputs_device(const double* d_displ, const double* d_q, const d
         if (!changed[0] && (changed[1] || changed[2])) {
             launch_update_inputs(A_, in, stream);
             CUDA_CHECK(cudaGetLastError());
-            // (evaluations asked for on the default stream run on the engine's own)
-            if (!stream) CUDA_CHECK(cudaStreamSynchronize(stream));
+            // the next evaluation may run on any stream, and the caller may write its
+            // buffers again
+            CUDA_CHECK(cudaStreamSynchronize(stream));
             nb_newer_on_device_ = true;
             bool disp = false;
             for (int r = 0; r < R_; r++) {
