@@ -229,7 +229,8 @@ int atm_batch_set_periodic_box_vectors(atm_batch_t b, int replica, const double*
  * positions) holds the replicas' positions back to back (host, nm); energies
  * (R), forces (sum n_r x 3, host) and results (R x ATM_NUM_RES) are nullable. */
 int atm_batch_evaluate(atm_batch_t b, const double* pos_all, double* energies, double* forces, double* results);
-/* Same with device pointers on the caller's CUDA stream (cudaStream_t as void*). */
+/* Same with device pointers on the caller's CUDA stream (cudaStream_t as void*; null: the
+ * legacy default stream), in order with what is queued there.  Waits for the evaluation. */
 int atm_batch_evaluate_device(atm_batch_t b, const double* d_pos_all, double* d_forces, double* d_results,
                               void* stream);
 /* R x R matrix of beta * (e0_r + W_s(u_r)): replica r's coordinates under

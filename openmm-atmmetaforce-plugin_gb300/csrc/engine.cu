@@ -1079,8 +1079,8 @@ std::string Engine::autotune(int trials, bool use_cache) {
                 const int t = sh.first;
                 const bool fu = sh.second;
                 apply_tuning(t, b, s != 0, fu);
-                run(nullptr, nullptr, h_pos_);  // uploads the staged positions (buffers may be new)
-                run(nullptr, nullptr);          // device graph capture + one warm evaluation
+                run(s_main_, nullptr, h_pos_);  // uploads the staged positions (buffers may be new)
+                run(s_main_, nullptr);          // device graph capture + one warm evaluation
                 CUDA_CHECK(cudaEventRecord(e0, s_main_));
                 for (int k = 0; k < trials; k++) CUDA_CHECK(cudaGraphLaunch(graph_dev_, s_main_));
                 CUDA_CHECK(cudaEventRecord(e1, s_main_));
@@ -1520,7 +1520,7 @@ static double* host_mapped(double* p) {
 // 1,500 atoms, 99 -> 95 at 12,000, 256 -> 252 at 46,000 and 1,323 -> 1,319 at 384,000 (the
 // reads hide behind one another, the copy's start-up did not).  A caller's own page-locked
 // buffer is still copied: the copy checks its extent, a kernel would not.
-void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos, bool host_results) {
+void Engine::run(cudaStream_t st, const double* d_pos, const double* h_pos, bool host_results) {
     const bool direct = h_pos && h_pos == h_pos_;
     struct Reset {  // (the next evaluation may be another kind)
         Engine* e;
@@ -1539,12 +1539,11 @@ void Engine::run(cudaStream_t user, const double* d_pos, const double* h_pos, bo
     settle_params();
     for (int attempt = 0; attempt < 4; attempt++) {
         update_rep_table();
-        update_influence(user ? user : s_main_);
+        update_influence(st);
         // the control word is read when the evaluation runs (it follows the
         // synchronisation that ends every evaluation of this path)
         h_ctl_[0] = (force_build_ || skin_ <= 0.0) ? 1 : 0;
         force_build_ = false;
-        cudaStream_t st = user ? user : s_main_;
         if (direct) {
             h_io_[0] = host_mapped(h_pos_);
             h_ctl_[1] |= EVAL_HOST_POSITIONS;

@@ -185,9 +185,11 @@ private:
     void fetch_nonbonded_params();
     void refresh_param_tables();
     void settle_params();
+    // st: the stream the evaluation runs on, in order with the work queued there; null is the
+    // legacy default stream, not s_main_ (nothing on the default stream waits for that one).
     // h_pos: positions from page-locked host memory.  host_results (implied by h_pos): the
     // result records and the matrix also end in h_results_ / h_matrix_
-    void run(cudaStream_t user, const double* d_pos, const double* h_pos = nullptr, bool host_results = false);
+    void run(cudaStream_t st, const double* d_pos, const double* h_pos = nullptr, bool host_results = false);
     bool check_status_and_grow();
     void destroy_graphs();
 
