@@ -218,6 +218,7 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
     CUDA_CHECK(cudaStreamCreateWithPriority(&s_pme_, cudaStreamNonBlocking, prio_greatest));
     CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     CUDA_CHECK(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
+    CUDA_CHECK(cudaEventCreateWithFlags(&ev_adjoint_, cudaEventDisableTiming));
     CUDA_CHECK(cudaMallocHost(&h_pos_, sizeof(double) * 3 * (size_t)n_in_));
     CUDA_CHECK(cudaMallocHost(&h_forces_, sizeof(double) * 3 * (size_t)n_in_));
     CUDA_CHECK(cudaMallocHost(&h_results_, sizeof(double) * NUM_RES * (size_t)R_));
@@ -266,6 +267,7 @@ Engine::~Engine() {
     cudaFreeHost(h_inputs_);
     if (ev_fork_) cudaEventDestroy(ev_fork_);
     if (ev_join_) cudaEventDestroy(ev_join_);
+    if (ev_adjoint_) cudaEventDestroy(ev_adjoint_);
     if (s_main_) cudaStreamDestroy(s_main_);
     if (s_pme_) cudaStreamDestroy(s_pme_);
 }
@@ -1393,6 +1395,17 @@ void Engine::settle_params() {
     params_pending_ = false;
 }
 
+// (The default stream is its own order, and is there to be recorded when another one
+// follows; a caller's stream may be gone by then.  Gradients in a caller's capture are
+// ordered by whoever launches it.)
+void Engine::after_adjoint(cudaStream_t st) {
+    if (!adjoint_pending_) return;
+    adjoint_pending_ = false;
+    if (!st && !adjoint_stream_) return;
+    if (!adjoint_stream_) CUDA_CHECK(cudaEventRecord(ev_adjoint_, adjoint_stream_));
+    CUDA_CHECK(cudaStreamWaitEvent(st, ev_adjoint_, 0));
+}
+
 void Engine::upload_params(cudaStream_t st) {
     if (h_params_sent_.size() == param_bytes_ && std::memcmp(h_params_sent_.data(), h_params_, param_bytes_) == 0) return;
     CUDA_CHECK(cudaMemcpyAsync(d_params_, h_params_, param_bytes_, cudaMemcpyHostToDevice, st));
@@ -1537,6 +1550,7 @@ void Engine::run(cudaStream_t st, const double* d_pos, const double* h_pos, bool
         alloc_device();
     }
     settle_params();
+    after_adjoint(st);
     for (int attempt = 0; attempt < 4; attempt++) {
         update_rep_table();
         update_influence(st);
@@ -1926,8 +1940,16 @@ void Engine::backward(const double* d_g, double* d_dx, double* d_dd, double* d_d
     if (!layout_ready_) throw Error(3, "backward() needs a preceding evaluation");
     if (!adjoint_ && (d_dq || d_dsig || d_deps))
         throw Error(3, "Charge/sigma/epsilon gradients need a batch created with Adjoint=1");
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (stream) CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
+    const bool capturing = capture != cudaStreamCaptureStatusNone;
+    if (!capturing) after_adjoint(stream);  // (one event stands for all of them)
     launch_adjoint(A_, d_g, d_dx, d_dd, d_dq, d_dsig, d_deps, d_dpar, stream);
     CUDA_CHECK(cudaGetLastError());
+    if (capturing) return;
+    if (stream) CUDA_CHECK(cudaEventRecord(ev_adjoint_, stream));
+    adjoint_stream_ = stream;
+    adjoint_pending_ = true;
 }
 
 }  // namespace atm

@@ -185,6 +185,8 @@ private:
     void fetch_nonbonded_params();
     void refresh_param_tables();
     void settle_params();
+    // Work on st that writes what the gradients read follows them.
+    void after_adjoint(cudaStream_t st);
     // st: the stream the evaluation runs on, in order with the work queued there; null is the
     // legacy default stream, not s_main_ (nothing on the default stream waits for that one).
     // h_pos: positions from page-locked host memory.  host_results (implied by h_pos): the
@@ -302,6 +304,10 @@ private:
 
     cudaStream_t s_main_ = nullptr, s_pme_ = nullptr;
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
+    // the last gradients, which may still be read from the force sums on adjoint_stream_
+    cudaEvent_t ev_adjoint_ = nullptr;
+    cudaStream_t adjoint_stream_ = nullptr;
+    bool adjoint_pending_ = false;
     // without and with host results; without any output
     cudaGraphExec_t graph_dev_ = nullptr, graph_res_ = nullptr, graph_lean_ = nullptr;
     std::vector<KernelTime> times_;

@@ -43,3 +43,36 @@ def test_positions_queued_on_the_stream_are_evaluated(own_stream):
     torch.cuda.synchronize()
     assert np.array_equal(before.cpu().numpy(), want[0])
     assert np.array_equal(after.cpu().numpy(), want[1])
+
+
+@pytest.mark.parametrize("second", ["host", "default", "side"])
+def test_gradients_are_those_of_the_evaluation_before_them(second):
+    """Gradients queued behind 10 ms of other work, and an evaluation of other positions
+    asked for on another stream meanwhile; gradients on two streams before it."""
+    case = _case(32)
+    batch = atm.ReplicaBatch([atm.system_from_case(case)[0]], 0, {"DifferencePath": 1, "Adjoint": 1})
+    first = torch.as_tensor(case.pos, device="cuda")
+    moved = first + 0.01 * torch.cos(torch.arange(first.numel(), device="cuda", dtype=torch.float64)).reshape(-1, 3)
+    g = torch.ones(1, dtype=torch.float64, device="cuda")
+    f = torch.empty_like(first)
+    r = torch.empty(1, NUM_RES, dtype=torch.float64, device="cuda")
+    batch.evaluate(case.pos)
+    want = batch.backward()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream() if second != "side" else torch.cuda.default_stream()]
+    dx = [torch.zeros_like(first) for _ in streams]
+    dq = [torch.zeros(case.n, dtype=torch.float64, device="cuda") for _ in streams]
+    torch.cuda.synchronize()
+    for k, s in enumerate(streams):
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(BUSY)
+        batch.backwardDevice(g.data_ptr(), dx[k].data_ptr(), d_dq=dq[k].data_ptr(), stream=s.cuda_stream)
+    if second == "host":
+        batch.evaluate(moved.cpu().numpy())
+    else:
+        s = torch.cuda.Stream() if second == "side" else torch.cuda.default_stream()
+        batch.evaluateDevice(moved.data_ptr(), f.data_ptr(), r.data_ptr(), s.cuda_stream)
+    torch.cuda.synchronize()
+    for k in range(2):
+        assert np.array_equal(dx[k].cpu().numpy(), want["positions"])
+        assert np.array_equal(dq[k].cpu().numpy(), want["charge"])
+    assert not np.array_equal(batch.backward()["positions"], want["positions"])
