@@ -1122,6 +1122,11 @@ void Engine::free_device() {
     d_allocs_.clear();
 }
 
+// What the buffers start with (copies from pageable memory, whose last part the device may
+// still be moving when the call returns, and fills) is there before a stream without an
+// order with the default one reads it.
+static void settle_uploads() { CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 template <typename T>
 static T* dalloc(std::vector<void*>& list, size_t n) {
     void* p = nullptr;
@@ -1316,6 +1321,7 @@ void Engine::alloc_device() {
     CUDA_CHECK(cudaMemset(a.status, 0, sizeof(Status)));
     CUDA_CHECK(cudaHostGetDevicePointer((void**)&a.h_status, h_status_, 0));
     a.h_results = a.h_matrix = nullptr;
+    settle_uploads();
 }
 
 // The dispersion correction of a replica at its box.  The coefficient depends on the
@@ -1884,6 +1890,7 @@ void Engine::set_inputs_device(const double* d_displ, const double* d_q, const d
                     CUDA_CHECK(cudaMemcpy(d_nb_ + k * (size_t)n_in_ + in_off_[r], v[k]->data(), sizeof(double) * s.n,
                                           cudaMemcpyHostToDevice));
             }
+            settle_uploads();
         }
         DeviceInputs in{d_displ, d_q, d_sig, d_eps, d_params, d_nb_, d_nb_ + n_in_, d_nb_ + 2 * (size_t)n_in_};
         CUDA_CHECK(cudaHostGetDevicePointer((void**)&in.changed, changed, 0));

@@ -523,6 +523,10 @@ T* md_upload(std::vector<void*>& list, const std::vector<T>& h) {
     return p;
 }
 
+// The driver's streams have no order with the default one: what copies from pageable memory
+// and fills put there is complete before a step reads it.
+void md_settle_uploads() { MD_CHECK(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -777,6 +781,7 @@ void MDDriver::upload_terms(const std::vector<const System*>& systems) {
     ke_d_ = md_alloc<double>(allocs_, R_);
     x_snap_ = md_alloc<double>(allocs_, 3 * (size_t)n_);
     v_snap_ = md_alloc<double>(allocs_, 3 * (size_t)n_);
+    md_settle_uploads();
 }
 
 MdDev MDDriver::dev_args() const {
@@ -835,6 +840,7 @@ MdDev MDDriver::dev_args() const {
 void MDDriver::set_positions(const double* pos) {
     MD_CHECK(cudaSetDevice(dev_));
     MD_CHECK(cudaMemcpy(x_, pos, sizeof(double) * 3 * (size_t)n_, cudaMemcpyHostToDevice));
+    md_settle_uploads();
     have_positions_ = true;
     forces_valid_ = false;
 }
@@ -842,6 +848,7 @@ void MDDriver::set_positions(const double* pos) {
 void MDDriver::set_velocities(const double* vel) {
     MD_CHECK(cudaSetDevice(dev_));
     MD_CHECK(cudaMemcpy(v_, vel, sizeof(double) * 3 * (size_t)n_, cudaMemcpyHostToDevice));
+    md_settle_uploads();
 }
 
 void MDDriver::set_velocities_to_temperature(double T, uint64_t seed) {
@@ -1041,6 +1048,7 @@ void MDDriver::step(int nsteps) {
     MD_CHECK(cudaStreamSynchronize(s_));
     if (failed) {
         MD_CHECK(cudaMemset(status_, 0, sizeof(int)));
+        md_settle_uploads();
         throw Error(10, "Constraints failed (SHAKE did not converge or SETTLE had no solution) in " +
                             std::to_string(failed) + " cluster-steps");
     }
