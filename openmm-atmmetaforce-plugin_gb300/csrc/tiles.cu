@@ -1404,21 +1404,32 @@ __global__ void __launch_bounds__(kTileThreads, MINB) k_tiles(Args a) {
 // evaluates them at once, while they are in L1 / L2; with kept lists (a skin) it
 // evaluates the row's tiles of the last build.  The finder's load-latency-bound
 // phases of some warps run beside the issue-bound pair loops of others on the
-// same SM.  Five CTAs of four warps per SM (102 registers, 45 KB of shared memory
-// each).
+// same SM.  Five CTAs of four warps per SM (96 registers, 43 KB of shared memory each;
+// the finder's candidate list takes the place of the j data, which a row's tiles need
+// only after it: with a place of its own four CTAs fit).  Four / five CTAs per SM, us of a
+// whole evaluation: 22 x 23,558 atoms 1,251 / 1,172, 8 x 60,000 1,304 / 1,239, 1 x 23,558
+// 150 / 107, 4 x 8,009 triclinic 513 / 451, 8 x 12,000 500 / 521 (five leave the PME chain
+// no registers beside them).
 constexpr int kFusedMinBlocks = 5;
+
+struct FusedWarpSmem {
+    int stage[kStageAtoms];
+    float4 ipos[32];
+    float4 buf[96];
+    int4 next_t[2];
+    int next_j[32];
+    int4 meta[32];
+};
+static_assert(kCandList * sizeof(int) <= sizeof(FusedWarpSmem::buf), "the candidate list takes the j data's place");
+static_assert(kFusedMinBlocks * (kFindWarps * sizeof(FusedWarpSmem) + 1024) <= 228 * 1024,
+              "the CTAs that the registers are budgeted for fit an SM's shared memory (1 KB of it reserved for each)");
 
 template <int METHOD, bool TRIC>
 __global__ void __launch_bounds__(kFindWarps * 32, kFusedMinBlocks) k_find_tiles(Args a) {
-    __shared__ int s_stage[kFindWarps][kStageAtoms];
-    __shared__ float4 s_ipos[kFindWarps][32];
-    __shared__ __align__(16) int s_cand[kFindWarps][kCandList];
-    __shared__ float4 s_buf[kFindWarps][96];
-    __shared__ int4 s_next_t[kFindWarps][2];
-    __shared__ int s_next_j[kFindWarps][32];
-    __shared__ int4 s_meta[kFindWarps][32];
+    __shared__ FusedWarpSmem s_warp[kFindWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const TileWarpSmem S{s_buf[w], s_next_t[w], s_next_j[w], s_meta[w]};
+    FusedWarpSmem& sm = s_warp[w];
+    const TileWarpSmem S{sm.buf, sm.next_t, sm.next_j, sm.meta};
     const bool build = a.status->rebuild != 0;
     if (build && a.skin_half2 > 0.f)  // the positions of this build, for the displacement test
         for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < a.NA; s += gridDim.x * blockDim.x)
@@ -1429,11 +1440,12 @@ __global__ void __launch_bounds__(kFindWarps * 32, kFusedMinBlocks) k_find_tiles
     while (k < a.nrows) {
         if (lane == 0) mine = nw < a.nrows ? nw + atomicAdd(&a.status->next_row, 1) : a.nrows;
         const int row = a.nrows - 1 - k;
-        if (build) find_row<TRIC>(a, row, lane, s_stage[w], s_ipos[w], s_cand[w]);
+        if (build) find_row<TRIC>(a, row, lane, sm.stage, sm.ipos, reinterpret_cast<int*>(sm.buf));
         __syncwarp();
         // the row's tiles (written by this warp just now, or by an earlier build)
         const int n = a.row_count[row], tb = a.row_tbase[row];
         if (n > 0 && tb + n <= a.tile_cap) tile_pairs<METHOD>(a, tb >> 1, (tb + n) >> 1, S);
+        __syncwarp();  // the j data are read before the next row's candidates take their place
         k = __shfl_sync(FULL_MASK, mine, 0);
     }
 }
