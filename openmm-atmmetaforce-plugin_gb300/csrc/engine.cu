@@ -1153,6 +1153,7 @@ void Engine::alloc_device() {
     free_device();
     Args& a = A_;
     a = Args{};
+    a.sms = sms_;
     a.R = R_;
     a.NA = NA_;
     a.NB = NB_;

@@ -223,6 +223,7 @@ struct Status {
 
 // Arguments shared by the kernels of one engine (passed by value).
 struct Args {
+    int sms;                  // SMs of the device
     // sizes
     int R, NA, NB, nrows, row_cap, tile_cap, n_in;
     int full;                 // 1: two full states, 0: state 1 + difference

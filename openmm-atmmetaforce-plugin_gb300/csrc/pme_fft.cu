@@ -280,11 +280,11 @@ __device__ __forceinline__ void stage_generic(const float2* src, float2* dst, co
     }
 }
 
-// nseq transforms of length N between buf0 and buf1 (same layout) following the
+// nseq transforms of the plan's length between buf0 and buf1 (same layout) following the
 // host's plan (plan: first stage | count << 24); returns 1 when the result is in
 // buf1, 0 when in buf0.  Every thread of the CTA calls it.
 template <bool INV>
-__device__ int fft_seqs(const Args& a, int plan, float2* buf0, float2* buf1, int N, int nseq, int ss, int es,
+__device__ int fft_seqs(const Args& a, int plan, float2* buf0, float2* buf1, int nseq, int ss, int es,
                         const float2* tw) {
     const FftStage* st = a.fft_stages + (plan & 0xffffff);
     const int nst = plan >> 24;
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(T, T == kWide ? 2 : 5) k_fft_zy(Args a) {
         b0[p * zs + z] = make_float2(re, im);
     }
     __syncthreads();
-    const int cz = fft_seqs<false>(a, R.fft_plan[2], b0, b1, K2, P, zs, 1, tw2);
+    const int cz = fft_seqs<false>(a, R.fft_plan[2], b0, b1, P, zs, 1, tw2);
     const float2* Z = cz ? b1 : b0;
     float2* S = cz ? b0 : b1;
     // Z = A + iB of two real rows: A_k = (Z_k + conj Z_-k) / 2, B_k = (Z_k - conj Z_-k) / (2i)
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(T, T == kWide ? 2 : 5) k_fft_zy(Args a) {
     }
     __syncthreads();
     float2* Zw = const_cast<float2*>(Z);
-    const int cy = fft_seqs<false>(a, R.fft_plan[1], S, Zw, K1, K2h, 1, K2h, tw1);
+    const int cy = fft_seqs<false>(a, R.fft_plan[1], S, Zw, K2h, 1, K2h, tw1);
     const float2* Y = cy ? Zw : S;
     float2* out = a.qcplx + R.cplx_off + (size_t)g * K0 * K1 * K2h + (size_t)ix * K2h;
 #pragma unroll 4
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(T, T == kWide ? 2 : 5) k_ifft_yz(Args a) {
     }
     cp_async_wait_all();
     __syncthreads();
-    const int cy = fft_seqs<true>(a, R.fft_plan[1], b0, b1, K1, K2h, 1, K2h, tw1);
+    const int cy = fft_seqs<true>(a, R.fft_plan[1], b0, b1, K2h, 1, K2h, tw1);
     const float2* S = cy ? b1 : b0;
     float2* Z = cy ? b0 : b1;
     // two rows' Hermitian half spectra as one complex row Z = A + iB (the
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(T, T == kWide ? 2 : 5) k_ifft_yz(Args a) {
     }
     __syncthreads();
     float2* Sw = const_cast<float2*>(S);
-    const int cz = fft_seqs<true>(a, R.fft_plan[2], Z, Sw, K2, P, zs, 1, tw2);
+    const int cz = fft_seqs<true>(a, R.fft_plan[2], Z, Sw, P, zs, 1, tw2);
     const float2* Zr = cz ? Sw : Z;
     float* G = a.qreal + R.real_off + (size_t)g * K0 * K1 * K2 + (size_t)ix * K1 * K2;
     if ((K2 & 3) == 0) {
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(T, T == kWide ? 2 : 4) k_fft_x_conv(Args a) {
     }
     cp_async_wait_all();
     __syncthreads();
-    int cur = fft_seqs<false>(a, R.fft_plan[0], b0, b1, K0, W, 1, W, tw0);
+    int cur = fft_seqs<false>(a, R.fft_plan[0], b0, b1, W, 1, W, tw0);
     float2* M = cur ? b1 : b0;
     // influence function G(m) = exp(-pi^2 m^2 / alpha^2) / (pi V m^2 B(m)), B the
     // B-spline moduli; the half spectrum counts kz in (0, K2/2) twice.  Each
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(T, T == kWide ? 2 : 4) k_fft_x_conv(Args a) {
         a.e_part_conv[2 * blockIdx.x + threadIdx.x] = t;
     }
     float2* other = cur ? b0 : b1;
-    cur = fft_seqs<true>(a, R.fft_plan[0], M, other, K0, W, 1, W, tw0);
+    cur = fft_seqs<true>(a, R.fft_plan[0], M, other, W, 1, W, tw0);
     const float2* out = cur ? other : M;
 #pragma unroll 4
     for (int w = threadIdx.x; w < K0 * W; w += blockDim.x) {
@@ -625,15 +625,7 @@ int fft_conv_smem_bytes(int K0, int nz) {
 }
 
 // points: of the largest plane, from its buffers' bytes
-static bool fft_wide(int planes, int points) {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
-    return planes <= 2 * sms && points >= kWideMin;
-}
+static bool fft_wide(const Args& a, int planes, int points) { return planes <= 2 * a.sms && points >= kWideMin; }
 
 template <typename K>
 static void launch_fft(K kernel, int threads, int ctas, int smem, const Args& a, cudaStream_t s) {
@@ -643,7 +635,7 @@ static void launch_fft(K kernel, int threads, int ctas, int smem, const Args& a,
 
 void launch_fft_forward(const Args& a, cudaStream_t s) {
     if (a.fft_plane_ctas <= 0) return;
-    if (fft_wide(a.fft_plane_ctas, a.fft_plane_smem / 16))
+    if (fft_wide(a, a.fft_plane_ctas, a.fft_plane_smem / 16))
         launch_fft(k_fft_zy<kWide>, kWide, a.fft_plane_ctas, a.fft_plane_smem, a, s);
     else
         launch_fft(k_fft_zy<kFftThreads>, kFftThreads, a.fft_plane_ctas, a.fft_plane_smem, a, s);
@@ -651,7 +643,7 @@ void launch_fft_forward(const Args& a, cudaStream_t s) {
 
 void launch_fft_conv(const Args& a, cudaStream_t s) {
     if (a.conv_ctas <= 0) return;
-    if (fft_wide(2 * a.conv_ctas, a.fft_conv_smem / 36))
+    if (fft_wide(a, 2 * a.conv_ctas, a.fft_conv_smem / 36))
         launch_fft(k_fft_x_conv<kWide>, kWide, a.conv_ctas, a.fft_conv_smem, a, s);
     else
         launch_fft(k_fft_x_conv<kFftThreads>, kFftThreads, a.conv_ctas, a.fft_conv_smem, a, s);
@@ -659,7 +651,7 @@ void launch_fft_conv(const Args& a, cudaStream_t s) {
 
 void launch_fft_inverse(const Args& a, cudaStream_t s) {
     if (a.fft_plane_ctas <= 0) return;
-    if (fft_wide(a.fft_plane_ctas, a.fft_plane_smem / 16))
+    if (fft_wide(a, a.fft_plane_ctas, a.fft_plane_smem / 16))
         launch_fft(k_ifft_yz<kWide>, kWide, a.fft_plane_ctas, a.fft_plane_smem, a, s);
     else
         launch_fft(k_ifft_yz<kFftThreads>, kFftThreads, a.fft_plane_ctas, a.fft_plane_smem, a, s);

@@ -765,15 +765,8 @@ int find_warps_per_sm() {
 }
 
 void launch_find(const Args& a, cudaStream_t s) {
-    static int per_sm = 0, sms = 0;
-    if (per_sm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_find<true>, kFindWarps * 32, 0);
-        if (per_sm < 1) per_sm = 1;
-    }
-    const int blocks = std::min(per_sm * sms, (a.nrows + kFindWarps - 1) / kFindWarps);
+    static const int per_sm = find_warps_per_sm() / kFindWarps;  // (several threads may record at once)
+    const int blocks = std::min(per_sm * a.sms, (a.nrows + kFindWarps - 1) / kFindWarps);
     if (a.any_tric)
         k_find<true><<<blocks, kFindWarps * 32, 0, s>>>(a);
     else
@@ -1450,18 +1443,16 @@ __global__ void __launch_bounds__(kFindWarps * 32, kFusedMinBlocks) k_find_tiles
     }
 }
 
+static int find_tiles_blocks_per_sm() {
+    int p4 = 0, p2 = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p4, k_find_tiles<4, true>, kFindWarps * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p2, k_find_tiles<2, true>, kFindWarps * 32, 0);
+    return std::max(1, std::min(p4, p2));
+}
+
 void launch_find_tiles(const Args& a, cudaStream_t s) {
-    static int per_sm = 0, sms = 0;
-    if (per_sm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int p4 = 0, p2 = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p4, k_find_tiles<4, true>, kFindWarps * 32, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p2, k_find_tiles<2, true>, kFindWarps * 32, 0);
-        per_sm = std::max(1, std::min(p4, p2));
-    }
-    const int blocks = std::min(per_sm * sms, (a.nrows + kFindWarps - 1) / kFindWarps);
+    static const int per_sm = find_tiles_blocks_per_sm();
+    const int blocks = std::min(per_sm * a.sms, (a.nrows + kFindWarps - 1) / kFindWarps);
     if (a.method == 4) {
         if (a.any_tric)
             k_find_tiles<4, true><<<blocks, kFindWarps * 32, 0, s>>>(a);
