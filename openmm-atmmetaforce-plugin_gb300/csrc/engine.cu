@@ -242,6 +242,7 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
     std::memset(h_pos_, 0, sizeof(double) * 3 * (size_t)n_in_);
     int per = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev_));
+    CUDA_CHECK(cudaDeviceGetAttribute(&smem_cta_, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev_));
     per = tiles_kernel_blocks_per_sm();
     if (per < 1) per = 1;
     max_tile_per_sm_ = per;
@@ -888,15 +889,13 @@ void Engine::build_layout() {
             }
         }
         // the hand-written transforms need a grid plane (two buffers) in shared memory
-        int smem_max = 0;
-        CUDA_CHECK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev_));
         fft_plane_smem_ = fft_conv_smem_ = 0;
         use_fft_ = true;
         for (int r = 0; r < R_; r++) {
             const RepDev& rd = rep_host_[r];
             const int b = fft_plane_smem_bytes(rd.K[1], rd.K[2]);
             fft_plane_smem_ = std::max(fft_plane_smem_, b);
-            if (b > smem_max - 1024) use_fft_ = false;
+            if (b > smem_cta_ - 1024) use_fft_ = false;
         }
         for (int r = 0; r < R_; r++) {
             RepDev& rd = rep_host_[r];
@@ -1154,6 +1153,7 @@ void Engine::alloc_device() {
     Args& a = A_;
     a = Args{};
     a.sms = sms_;
+    a.smem_cta = smem_cta_;
     a.R = R_;
     a.NA = NA_;
     a.NB = NB_;

@@ -225,7 +225,7 @@ private:
     bool layout_ready_ = false;
     bool profiling_ = false;
     int tile_grid_ = 0;
-    int sms_ = 0, max_tile_per_sm_ = 1;
+    int sms_ = 0, smem_cta_ = 0, max_tile_per_sm_ = 1;
     int tune_tile_per_sm_ = 0;     // 0: as many as fit
     static constexpr int kBrickAuto = -1;
     int tune_brick_ = kBrickAuto;  // spreading brick edge (grid points), 0: per atom; kBrickAuto: build_bricks' rule

@@ -864,9 +864,7 @@ void launch_spread(const Args& a, cudaStream_t s, bool with_exceptions) {
     }
     if (a.brick_ctas <= 0) return;
     const int bytes = spread_smem_bytes(a.brick_smem);
-    // opt in to more than 48 KB of dynamic shared memory (per device; this runs
-    // when the evaluation graph is recorded, not at every evaluation)
-    cudaFuncSetAttribute(k_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    allow_shared_memory(k_spread, a);
     k_spread<<<a.brick_ctas, kBrickThreads, bytes, s>>>(a);
 }
 

@@ -224,6 +224,7 @@ struct Status {
 // Arguments shared by the kernels of one engine (passed by value).
 struct Args {
     int sms;                  // SMs of the device
+    int smem_cta;             // shared memory a CTA may have on it (bytes)
     // sizes
     int R, NA, NB, nrows, row_cap, tile_cap, n_in;
     int full;                 // 1: two full states, 0: state 1 + difference
@@ -353,6 +354,17 @@ struct Args {
     double* h_results;        // or null
     double* h_matrix;         // or null
 };
+
+// Opts a kernel in to all the dynamic shared memory a CTA may have, whatever this launch
+// needs: the limit is the kernel's, not the launch's, so that a smaller one set by another
+// thread would take back what this thread's next launch needs.  (Per device; at recordings,
+// not at evaluations.)
+template <typename K>
+inline void allow_shared_memory(K kernel, const Args& a) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kernel) == cudaSuccess)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem_cta - (int)fa.sharedSizeBytes);
+}
 
 void launch_prepare(const Args& a, cudaStream_t s);
 void launch_find(const Args& a, cudaStream_t s);

@@ -629,7 +629,7 @@ static bool fft_wide(const Args& a, int planes, int points) { return planes <= 2
 
 template <typename K>
 static void launch_fft(K kernel, int threads, int ctas, int smem, const Args& a, cudaStream_t s) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_shared_memory(kernel, a);
     kernel<<<ctas, threads, smem, s>>>(a);
 }
 
