@@ -890,11 +890,13 @@ void Engine::build_layout() {
         }
         // the hand-written transforms need a grid plane (two buffers) in shared memory
         fft_plane_smem_ = fft_conv_smem_ = 0;
+        fft_plane_points_ = fft_conv_points_ = 0;
         use_fft_ = true;
         for (int r = 0; r < R_; r++) {
             const RepDev& rd = rep_host_[r];
             const int b = fft_plane_smem_bytes(rd.K[1], rd.K[2]);
             fft_plane_smem_ = std::max(fft_plane_smem_, b);
+            fft_plane_points_ = std::max(fft_plane_points_, fft_plane_points(rd.K[1], rd.K[2]));
             if (b > smem_cta_ - 1024) use_fft_ = false;
         }
         for (int r = 0; r < R_; r++) {
@@ -911,6 +913,7 @@ void Engine::build_layout() {
                 for (int ky = 0; ky < rd.K[1]; ky++)
                     for (int z0 = 0; z0 < K2h; z0 += nz) fft_conv_.push_back(make_int4(r, ky, z0, std::min(K2h, z0 + nz)));
                 fft_conv_smem_ = std::max(fft_conv_smem_, fft_conv_smem_bytes(rd.K[0], nz));
+                fft_conv_points_ = std::max(fft_conv_points_, rd.K[0] * nz);
                 rd.conv_cta_e = (int)fft_conv_.size();
             } else {
                 const long long per = 4096;
@@ -1282,6 +1285,8 @@ void Engine::alloc_device() {
         a.fft_plane_ctas = (int)fft_plane_.size();
         a.fft_plane = dupload(d_allocs_, fft_plane_);
         a.fft_plane_smem = fft_plane_smem_;
+        a.fft_plane_points = fft_plane_points_;
+        a.fft_conv_points = fft_conv_points_;
         a.fft_conv = dupload(d_allocs_, fft_conv_);
         a.fft_conv_smem = fft_conv_smem_;
         a.influence = use_fft_ ? dalloc<float>(d_allocs_, n_cplx_ / 2) : nullptr;

@@ -271,6 +271,7 @@ private:
     std::vector<int2> fft_plane_;
     std::vector<int4> fft_conv_;
     int fft_plane_smem_ = 0, fft_conv_smem_ = 0;
+    int fft_plane_points_ = 0, fft_conv_points_ = 0;
     bool infl_dirty_ = true;  // the influence-function table needs computing (new buffers or boxes)
     void update_influence(cudaStream_t st);
 

@@ -337,6 +337,8 @@ struct Args {
     int fft_plane_ctas;       // (grid, x-plane) CTAs of all replicas
     const int2* fft_plane;    //   (replica, grid * K0 + x)
     int fft_plane_smem;       // dynamic shared memory of a plane CTA (bytes)
+    int fft_plane_points;     // points of the largest plane, and of one grid's part of the largest x slab
+    int fft_conv_points;
     const int4* fft_conv;     // conv CTAs: (replica, ky, kz0, kz1)
     int fft_conv_smem;
     float* influence;         // influence function per replica, [ky][x][kz] at cplx_off / 2
@@ -378,6 +380,7 @@ void launch_gather(const Args& a, cudaStream_t s);
 void launch_fft_forward(const Args& a, cudaStream_t s);
 void launch_fft_conv(const Args& a, cudaStream_t s);
 void launch_fft_inverse(const Args& a, cudaStream_t s);
+int fft_plane_points(int K1, int K2);
 int fft_plane_smem_bytes(int K1, int K2);
 // Stages of a 1D transform of length N (twiddles tw) appended to out, the roots of its prime
 // stages to roots; returns first | count << 24.

@@ -35,16 +35,20 @@
 namespace atm {
 
 // Threads of a CTA of the three kernels: kFftThreads, or twice as many (kWide) where the
-// time is a CTA's own chain of loops: planes of at least kWideMin points and at most two
+// time is a CTA's own chain of loops: planes of at least kWideMin points (of the larger of
+// the two layouts of a plane; of the x slabs, grid points per slab and grid) and at most two
 // per SM (x slabs, whose CTA holds two planes: one).  us of 20 MD steps, 256 / 512 threads:
 // 1 x 23,558 atoms (112 planes of 56 x 29 points) 2,936 / 2,808, 2 x 23,558 3,896 / 3,787,
 // 1 x 46,001 (69 points) 4,930 / 4,127, 2 x 46,001 7,240 / 6,742; a state of one 46,001-atom
 // system 414 / 386.  Smaller or more planes lose: 4 x 5,000 (288 of 36 x 19) 3,304 / 3,500,
 // 3 x 12,000 (270 of 45 x 23) 3,331 / 3,437, 4 x 8,009 (352) 240 / 249 a pass, 22 x 23,558
-// 973 / 1,036.
+// 973 / 1,036.  Around the line, an evaluation of one 12,000 / one 23,558-atom system: 1,200
+// points (48) 78 / 77 and 98.5 / 99.5, 1,300 (50) 77 / 74 and 98.9 / 101.2, 1,404 (52) 107 / 95
+// and 120 / 110, 1,431 (53) 162 / 115 and 182 / 136, 1,485 (55 x 52) 109 / 93 and 116 / 108,
+// 1,512 (54) 82 / 80 and 99.8 / 100.2.
 constexpr int kFftThreads = 256;
 constexpr int kWide = 2 * kFftThreads;
-constexpr int kWideMin = 1500;
+constexpr int kWideMin = 1400;
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -581,9 +585,13 @@ void launch_influence(float* G, const float* moduli, const int* mod_off, const i
                                       K[2], recip[0], recip[1], recip[2], recip[3], recip[4], recip[5], volume, alpha);
 }
 
-int fft_plane_smem_bytes(int K1, int K2) {
+int fft_plane_points(int K1, int K2) {
     const int P = (K1 + 1) / 2, K2h = K2 / 2 + 1, zs = K2 | 1;
-    const int plane = ((P * zs > K1 * K2h ? P * zs : K1 * K2h) + 1) & ~1;
+    return P * zs > K1 * K2h ? P * zs : K1 * K2h;
+}
+
+int fft_plane_smem_bytes(int K1, int K2) {
+    const int plane = (fft_plane_points(K1, K2) + 1) & ~1;
     return (int)sizeof(float2) * (2 * plane + K1 + K2);
 }
 
@@ -624,7 +632,7 @@ int fft_conv_smem_bytes(int K0, int nz) {
     return (int)sizeof(float2) * (2 * K0 * 2 * nz + K0) + (int)sizeof(float) * ((K0 * nz + 1) & ~1);
 }
 
-// points: of the largest plane, from its buffers' bytes
+// points: of the largest plane or slab
 static bool fft_wide(const Args& a, int planes, int points) { return planes <= 2 * a.sms && points >= kWideMin; }
 
 template <typename K>
@@ -635,7 +643,7 @@ static void launch_fft(K kernel, int threads, int ctas, int smem, const Args& a,
 
 void launch_fft_forward(const Args& a, cudaStream_t s) {
     if (a.fft_plane_ctas <= 0) return;
-    if (fft_wide(a, a.fft_plane_ctas, a.fft_plane_smem / 16))
+    if (fft_wide(a, a.fft_plane_ctas, a.fft_plane_points))
         launch_fft(k_fft_zy<kWide>, kWide, a.fft_plane_ctas, a.fft_plane_smem, a, s);
     else
         launch_fft(k_fft_zy<kFftThreads>, kFftThreads, a.fft_plane_ctas, a.fft_plane_smem, a, s);
@@ -643,7 +651,7 @@ void launch_fft_forward(const Args& a, cudaStream_t s) {
 
 void launch_fft_conv(const Args& a, cudaStream_t s) {
     if (a.conv_ctas <= 0) return;
-    if (fft_wide(a, 2 * a.conv_ctas, a.fft_conv_smem / 36))
+    if (fft_wide(a, 2 * a.conv_ctas, a.fft_conv_points))
         launch_fft(k_fft_x_conv<kWide>, kWide, a.conv_ctas, a.fft_conv_smem, a, s);
     else
         launch_fft(k_fft_x_conv<kFftThreads>, kFftThreads, a.conv_ctas, a.fft_conv_smem, a, s);
@@ -651,7 +659,7 @@ void launch_fft_conv(const Args& a, cudaStream_t s) {
 
 void launch_fft_inverse(const Args& a, cudaStream_t s) {
     if (a.fft_plane_ctas <= 0) return;
-    if (fft_wide(a, a.fft_plane_ctas, a.fft_plane_smem / 16))
+    if (fft_wide(a, a.fft_plane_ctas, a.fft_plane_points))
         launch_fft(k_ifft_yz<kWide>, kWide, a.fft_plane_ctas, a.fft_plane_smem, a, s);
     else
         launch_fft(k_ifft_yz<kFftThreads>, kFftThreads, a.fft_plane_ctas, a.fft_plane_smem, a, s);
