@@ -212,7 +212,7 @@ Engine::Engine(std::vector<ReplicaSpec> reps, int device, bool full_mode, bool a
 
     CUDA_CHECK(cudaSetDevice(dev_));
     CUDA_CHECK(cudaStreamCreateWithFlags(&s_main_, cudaStreamNonBlocking));
-    // the PME chain's CTAs go first wherever one ends (Engine::tile_launch_grid)
+    // the PME chain's CTAs go first wherever one ends (Engine::tile_launch)
     int prio_least = 0, prio_greatest = 0;
     CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest));
     CUDA_CHECK(cudaStreamCreateWithPriority(&s_pme_, cudaStreamNonBlocking, prio_greatest));
@@ -1010,8 +1010,8 @@ void Engine::apply_tuning(int tile_per_sm, int brick, bool pme_stream, bool fuse
     tune_fused_ = fused;
     A_.fused = fused ? 1 : 0;
     tile_grid_ = sms_ * std::min(std::max(1, tile_per_sm), max_tile_per_sm_);
-    A_.tile_dynamic = tile_dynamic();
-    A_.tile_wide = tile_grid_ <= 3 * sms_ ? 1 : 0;
+    A_.tile_dynamic = tile_launch().dynamic;
+    A_.tile_wide = tile_launch().wide;
     if (rebuild && layout_ready_ && method_ == NonbondedForce::PME) {
         build_bricks();
         alloc_device();
@@ -1072,11 +1072,23 @@ std::string Engine::autotune(int trials, bool use_cache) {
     cudaEvent_t e0, e1;
     CUDA_CHECK(cudaEventCreate(&e0));
     CUDA_CHECK(cudaEventCreate(&e1));
-    // separate list and pair-tile kernels at 4, 3, 2 pair-tile CTAs per SM, then the
-    // fused kernel (its CTAs per SM are fixed)
+    // separate list and pair-tile kernels at 4, 3, 2 pair-tile CTAs per SM, as far as they
+    // are launched differently (a small list in one pass takes as many CTAs at 3 as at 2),
+    // then the fused kernel (its CTAs per SM are fixed)
     std::vector<std::pair<int, bool>> shapes;
-    for (int t = max_tile_per_sm_; t >= 2 && t >= max_tile_per_sm_ - 2; t--) shapes.push_back({t, false});
+    std::map<std::array<int, 3>, int> launches;
+    for (int t = max_tile_per_sm_; t >= 2 && t >= max_tile_per_sm_ - 2; t--) {
+        tile_grid_ = sms_ * t;
+        const TileLaunch l = tile_launch();
+        if (launches.emplace(std::array<int, 3>{l.dynamic, l.wide, l.grid}, t).second) shapes.push_back({t, false});
+    }
     shapes.push_back({max_tile_per_sm_, true});
+    auto shape_name = [&](bool fused) -> std::string {  // of the tuning applied
+        if (fused) return "fused lists+tiles";
+        const TileLaunch l = tile_launch();
+        if (l.grid == tile_grid_) return "tiles/SM=" + std::to_string(tile_grid_ / sms_);
+        return std::string("tiles in one pass, ") + (l.wide ? "80" : "64") + " registers";
+    };
     for (const auto& sh : shapes)
         for (int b : bricks)
             for (int s : pmes) {
@@ -1092,11 +1104,7 @@ std::string Engine::autotune(int trials, bool use_cache) {
                 float ms = 0;
                 CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
                 ms /= trials;
-                if (fu)
-                    rep << "fused lists+tiles";
-                else
-                    rep << "tiles/SM=" << t;
-                rep << " brick=" << b << " pme_stream=" << s << " : " << ms << " ms\n";
+                rep << shape_name(fu) << " brick=" << b << " pme_stream=" << s << " : " << ms << " ms\n";
                 if (ms < best) {
                     best = ms;
                     bt = t;
@@ -1108,8 +1116,7 @@ std::string Engine::autotune(int trials, bool use_cache) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     apply_tuning(bt, bb, bs, bf);
-    rep << "chosen: " << (bf ? "fused lists+tiles" : "tiles/SM=" + std::to_string(bt)) << " brick=" << bb
-        << " pme_stream=" << bs << " (" << best << " ms)\n";
+    rep << "chosen: " << shape_name(bf) << " brick=" << bb << " pme_stream=" << bs << " (" << best << " ms)\n";
     std::ofstream f(cache_path(), std::ios::app);
     if (f) f << tuning_key() << "\t" << bt << " " << bb << " " << (bs ? 1 : 0) << " " << (bf ? 1 : 0) << "\n";
     return rep.str();
@@ -1169,8 +1176,8 @@ void Engine::alloc_device() {
     a.rc2 = cutoff2();
     a.rcl2 = list_cutoff2();
     a.skin_half2 = (float)(0.25 * skin_ * skin_);
-    a.tile_dynamic = tile_dynamic();
-    a.tile_wide = tile_grid_ <= 3 * sms_ ? 1 : 0;
+    a.tile_dynamic = tile_launch().dynamic;
+    a.tile_wide = tile_launch().wide;
     a.fused = tune_fused_ ? 1 : 0;
     a.alpha = (float)alpha_;
     a.krf = (float)krf_;
@@ -1379,14 +1386,13 @@ void Engine::update_rep_table() {
 // 23,558 atoms, 50 MD steps 7200 / 6630, PME context 285 / 281; 8 x 12,000 (3,016 rows,
 // 4,864 warps), 20 MD steps 7340 / 6750, boxes of three sizes 379 / 372; 22 x 23,558
 // (16,280 rows) 1006 / 1031, 8 x 60,000 1184 / 1230.
-int Engine::tile_dynamic() const {
-    const long long warps = (long long)tile_grid_ * (kTileThreads / 32);
-    return nrows_ / row_parts_ >= warps ? 1 : 0;
-}
-
-int Engine::tile_launch_grid() const {
-    if (A_.tile_dynamic) return tile_grid_;
-    return std::max(tile_grid_, (int)(4.5 * (nrows_ / row_parts_)));
+Engine::TileLaunch Engine::tile_launch() const {
+    const int rows = nrows_ / row_parts_;
+    TileLaunch l;
+    l.dynamic = rows >= (long long)tile_grid_ * (kTileThreads / 32) ? 1 : 0;
+    l.wide = tile_grid_ <= 3 * sms_ ? 1 : 0;
+    l.grid = l.dynamic ? tile_grid_ : std::max(tile_grid_, (int)(4.5 * rows));
+    return l;
 }
 
 int Engine::launches_per_eval() const {
@@ -1461,7 +1467,7 @@ void Engine::record(cudaStream_t st, const Args& a, bool output) {
         launch_find_tiles(a, st);
     } else {
         launch_find(a, st);
-        launch_tiles(a, tile_launch_grid(), st);
+        launch_tiles(a, tile_launch().grid, st);
     }
     if ((pme && tune_pme_stream_) || exc_beside) CUDA_CHECK(cudaStreamWaitEvent(st, ev_join_, 0));
     launch_finalize(a, st);
@@ -1606,7 +1612,7 @@ void Engine::run(cudaStream_t st, const double* d_pos, const double* h_pos, bool
             } else {
                 launch_find(a, st);
                 mark("find");
-                launch_tiles(a, tile_launch_grid(), st);
+                launch_tiles(a, tile_launch().grid, st);
                 mark("tiles");
             }
             launch_exceptions(a, st);

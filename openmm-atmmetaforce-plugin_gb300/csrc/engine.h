@@ -147,8 +147,12 @@ public:
     void set_profiling(bool on) { profiling_ = on; }
     const std::vector<KernelTime>& kernel_times() const { return times_; }
     int launches_per_eval() const;
-    int tile_dynamic() const;
-    int tile_launch_grid() const;
+    // How the pair tiles are launched at tile_grid_: from a counter or in one pass, in the
+    // 80-register variant or the 64-register one, and the CTAs.
+    struct TileLaunch {
+        int dynamic, wide, grid;
+    };
+    TileLaunch tile_launch() const;
     // tiles of the last evaluation, tile rows, and the largest row
     void stats(int* tiles, int* rows, int* max_row) const {
         if (tiles) *tiles = last_tiles_;

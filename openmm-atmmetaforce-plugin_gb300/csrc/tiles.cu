@@ -1380,7 +1380,7 @@ __global__ void __launch_bounds__(kTileThreads, MINB) k_tiles(Args a) {
     // lists: pairs handed out kTileGrab at a time from a counter (the next grab
     // requested before the current pairs are processed), so that warps finish
     // together.  Small lists (about a pair per warp): warp w takes pairs w, w + nw, ...
-    // (DYN, chosen by the host from the size of the row list, Engine::tile_dynamic)
+    // (DYN, chosen by the host from the size of the row list, Engine::tile_launch)
     int mine = 0;
     if (DYN && lane == 0) mine = atomicAdd(&a.status->next_tile, kTileGrab);
     int cur = DYN ? __shfl_sync(FULL_MASK, mine, 0) : ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
