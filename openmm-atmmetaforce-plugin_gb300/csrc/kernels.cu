@@ -80,6 +80,7 @@ __device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDe
 
 // The box around the eight blocks of a CTA (one warp; box: their centres and half
 // extents, rep: their replicas, -1: none), at the images nearest the first one's centre.
+// No number when a block's is none (its first atom's position is none).
 __device__ __forceinline__ void octet_bbox(const Args& a, const float4 (*box)[2], const int* rep, int lane, float4* c,
                                            float4* h) {
     const RepDev& R = a.reps[rep[0]];
@@ -91,12 +92,12 @@ __device__ __forceinline__ void octet_bbox(const Args& a, const float4 (*box)[2]
     float lx = dx - hb.x, ly = dy - hb.y, lz = dz - hb.z, hx = dx + hb.x, hy = dy + hb.y, hz = dz + hb.z;
 #pragma unroll
     for (int o = 1; o <= 4; o <<= 1) {
-        lx = fminf(lx, __shfl_xor_sync(FULL_MASK, lx, o));
-        ly = fminf(ly, __shfl_xor_sync(FULL_MASK, ly, o));
-        lz = fminf(lz, __shfl_xor_sync(FULL_MASK, lz, o));
-        hx = fmaxf(hx, __shfl_xor_sync(FULL_MASK, hx, o));
-        hy = fmaxf(hy, __shfl_xor_sync(FULL_MASK, hy, o));
-        hz = fmaxf(hz, __shfl_xor_sync(FULL_MASK, hz, o));
+        lx = bound_min(lx, __shfl_xor_sync(FULL_MASK, lx, o));
+        ly = bound_min(ly, __shfl_xor_sync(FULL_MASK, ly, o));
+        lz = bound_min(lz, __shfl_xor_sync(FULL_MASK, lz, o));
+        hx = bound_max(hx, __shfl_xor_sync(FULL_MASK, hx, o));
+        hy = bound_max(hy, __shfl_xor_sync(FULL_MASK, hy, o));
+        hz = bound_max(hz, __shfl_xor_sync(FULL_MASK, hz, o));
     }
     if (lane == 0) {
         *c = make_float4(c0.x + 0.5f * (lx + hx), c0.y + 0.5f * (ly + hy), c0.z + 0.5f * (lz + hz), 0.f);

@@ -12,6 +12,8 @@
 #include <vector>
 #include <cuda_runtime.h>
 
+#include "boxes.h"
+
 namespace atm {
 
 constexpr int kTile = 32;

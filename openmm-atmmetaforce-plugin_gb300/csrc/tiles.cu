@@ -109,13 +109,6 @@ __device__ __forceinline__ void min_image_t(float& x, float& y, float& z, const 
     }
 }
 
-__device__ __forceinline__ float box_gap2(float dx, float dy, float dz, float hx, float hy, float hz) {
-    dx = fmaxf(0.f, fabsf(dx) - hx);
-    dy = fmaxf(0.f, fabsf(dy) - hy);
-    dz = fmaxf(0.f, fabsf(dz) - hz);
-    return dx * dx + dy * dy + dz * dz;
-}
-
 // Are two blocks' bounding boxes closer than the cutoff?  The centres' minimum
 // image (per axis, exact for orthorhombic boxes); triclinic rows that need
 // per-pair images (all_images) take the closest of the 125 images around it.
