@@ -622,7 +622,8 @@ void Engine::layout_replica(int r, RepLayout& L) const {
 // Runs f(0 .. n - 1) on up to 16 threads; the first exception is thrown again here.
 template <typename F>
 static void parallel_for(int n, const F& f) {
-    const int nt = std::min({n, 16, (int)std::max(1u, std::thread::hardware_concurrency())});
+    static const int cores = (int)std::max(1u, std::thread::hardware_concurrency());  // (a look-up of some 10 us)
+    const int nt = std::min({n, 16, cores});
     if (nt <= 1) {
         for (int k = 0; k < n; k++) f(k);
         return;
@@ -1667,18 +1668,12 @@ static bool is_pinned(const void* p) {
 // Host copy split over a few threads (a single core moves ~10-20 GB/s).
 static void par_memcpy(void* dst, const void* src, size_t bytes) {
     const size_t kMin = size_t(4) << 20;
-    int nt = (int)std::min<size_t>(8, std::max<size_t>(1, bytes / kMin));
-    if (nt <= 1) {
-        std::memcpy(dst, src, bytes);
-        return;
-    }
-    std::vector<std::thread> th;
-    size_t chunk = (bytes + nt - 1) / nt;
-    for (int t = 0; t < nt; t++) {
-        size_t b = (size_t)t * chunk, e = std::min(bytes, b + chunk);
-        if (b < e) th.emplace_back([=] { std::memcpy((char*)dst + b, (const char*)src + b, e - b); });
-    }
-    for (auto& x : th) x.join();
+    const int nt = (int)std::min<size_t>(8, std::max<size_t>(1, bytes / kMin));
+    const size_t chunk = (bytes + nt - 1) / nt;
+    parallel_for(nt, [&](int t) {
+        const size_t b = (size_t)t * chunk, e = std::min(bytes, b + chunk);
+        if (b < e) std::memcpy((char*)dst + b, (const char*)src + b, e - b);
+    });
 }
 
 void Engine::evaluate_host(const double* pos, double* energies, double* forces, double* results, double* matrix) {
