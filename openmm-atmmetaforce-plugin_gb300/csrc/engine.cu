@@ -1386,7 +1386,13 @@ void Engine::update_rep_table() {
 // persistent CTAs fill every SM until the list is done.  Persistent / one pass, us:
 // 23,558 atoms, 50 MD steps 7200 / 6630, PME context 285 / 281; 8 x 12,000 (3,016 rows,
 // 4,864 warps), 20 MD steps 7340 / 6750, boxes of three sizes 379 / 372; 22 x 23,558
-// (16,280 rows) 1006 / 1031, 8 x 60,000 1184 / 1230.
+// (16,280 rows) 1006 / 1031, 8 x 60,000 1184 / 1230.  Around the line, an evaluation of
+// R x 12,000 atoms: 4,158 rows 305 / 295, 4,536 326 / 317, 4,914 345 / 341, 5,292 365 / 363,
+// 6,048 417 / 411, 9,828 654 / 658; R x 23,558: 4,434 rows 332 / 321, 5,173 374 / 366, 7,390
+// 515 / 512, 9,607 621 / 620; R x 60,000: 3,756 rows 354 / 347, 5,634 495 / 477, 7,512
+// 570 / 588.  Boxes so small that every pair needs its own image have more and longer tiles
+// a row and cross over sooner: R x 5,000: 3,816 rows 403 / 395, 4,452 456 / 470, 4,770
+// 480 / 512, 5,088 509 / 549, 6,996 672 / 747.
 Engine::TileLaunch Engine::tile_launch() const {
     const int rows = nrows_ / row_parts_;
     TileLaunch l;

@@ -44,8 +44,9 @@ __device__ __forceinline__ float wrapf(float x, float L, float iL) { return x - 
 // prepare: one warp per block
 // ---------------------------------------------------------------------------
 // Bounding box of a block (minimum image relative to its first atom); h.w receives
-// the number of real (non-padding) atoms of the block; box: c and h again.  With hc, also the boxes of its
-// two halves, whose h.w receives the largest distance of an atom from the box centre.
+// the number of real (non-padding) atoms of the block; box: c and h again.  With hc, also
+// the boxes of its two halves, whose h.w receives the largest distance of an atom from the
+// box centre.
 __device__ __forceinline__ void warp_bbox(float x, float y, float z, const RepDev& R, int b, float4* c, float4* h,
                                           float4* hc, float4* hh, int lane, int nreal, float4* box) {
     float x0 = __shfl_sync(FULL_MASK, x, 0), y0 = __shfl_sync(FULL_MASK, y, 0), z0 = __shfl_sync(FULL_MASK, z, 0);
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(Args a, int nprep) {
             float dx = x - r.x, dy = y - r.y, dz = z - r.z;
             min_image3(dx, dy, dz, R);
             float d2 = dx * dx + dy * dy + dz * dz;
-    #pragma unroll
+#pragma unroll
             for (int o = 16; o > 0; o >>= 1) d2 = fmaxf(d2, __shfl_xor_sync(FULL_MASK, d2, o));
             // non-negative floats order as their bit patterns
             if (lane == 0) atomicMax(&a.status->disp2, __float_as_uint(d2));
@@ -775,7 +776,6 @@ __global__ void __launch_bounds__(kBrickThreads) k_spread(Args a) {
 constexpr int kSpreadAtomWarps = 8;
 constexpr int kSpreadAtoms = 8;
 
-//
 // The first nexc CTAs evaluate the exceptions, which the PME chain would otherwise
 // wait for (5 of its 60 us on one 23,558-atom box).
 static_assert(kExcThreads == kSpreadAtomWarps * 32, "exceptions and spreading share a launch");

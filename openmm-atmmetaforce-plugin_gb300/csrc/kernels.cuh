@@ -92,7 +92,6 @@ enum Res {
     RES_DL1, RES_DL2, RES_DALPHA, RES_DU0, RES_DW0, RES_STATUS, RES_DWDU, NUM_RES
 };
 
-// Per-replica constants and offsets (device copy refreshed every evaluation).
 // One Stockham stage of a 1D transform of length N: radix R, Ns the product of
 // the earlier stages' radices, nb = N / R butterflies, step = N / (Ns R) (the
 // twiddle exponent's stride), mNs = ceil(2^32 / Ns) for the division by Ns.
@@ -103,6 +102,8 @@ struct FftStage {
     int pad[2];
 };
 
+// Per-replica constants and offsets (the device's copy follows at the next evaluation after a
+// change; new buffers hold none before their first).
 struct RepDev {
     float box[4];      // L (x,y,z), unused
     float ibox[4];     // 1/L

@@ -898,11 +898,12 @@ void MDDriver::set_recording(int interval, int capacity) {
     }
 }
 
-// Device-to-device copies of the current evaluation into the ring (no host wait).
+// Whether the current evaluation goes into the ring.
 bool MDDriver::record_due() const {
     return rec_interval_ > 0 && step_ % rec_interval_ == 0 && step_ != rec_last_step_;
 }
 
+// Device-to-device copies of the current evaluation into the ring (no host wait).
 void MDDriver::record_step() {
     if (!record_due()) return;
     const int slot = (int)(rec_count_ % rec_cap_);
