@@ -226,9 +226,8 @@ __device__ __forceinline__ int exact_cut_half(const Args& a, const RepDev& R, in
     const __half2 thr = __float2half2_rn(rcm * rcm);
     const uint4* ih = reinterpret_cast<const uint4*>(s_ipos);
     const unsigned lt = (1u << lane) - 1u;
-    // atoms per lane, which share each i atom's read (1 / 2 / 3: 163 / 159 / 161 M warp
-    // instructions, 254 / 244 / 251 us on 22 x 23,558 atoms; 170 M and 258 us with a
-    // comparison per pair and an exit when every lane had a hit)
+    // atoms per lane, which share each i atom's read (1 / 2 / 3: 147 / 145 / 147 M warp
+    // instructions, 231 / 225 / 250 us on 22 x 23,558 atoms, 201 / 195 / 218 us on 8 x 60,000)
     constexpr int kPer = 2;
     int kept = from;
     for (int g = from; g < natom; g += 32 * kPer) {
@@ -349,9 +348,10 @@ __device__ __noinline__ int exact_cut(const Args& a, const RepDev& R, int kind, 
 // Which blocks are tested: rows in one part first test the boxes of octets of blocks
 // (consecutive along the Hilbert curve, so compact), 32 at once, and then the blocks of
 // the octets within the cutoff, four octets at once; rows in parts test their blocks in
-// strides, 32 at once.  Bound by instruction issue (62 % active): octets take 22 x
-// 23,558 atoms from 159 to 148 M warp instructions, and the candidate tests off the time
-// of long rows: 8 x 60,000 atoms 311 -> 216 us, 22 x 23,558 244 -> 238.
+// strides, 32 at once.  Bound by instruction issue (63 % active): the octets and the exact
+// cut's two atoms per lane take 22 x 23,558 atoms from 170 to 148 M warp instructions (the
+// list to 145 M), the octets the candidate tests off the time of long rows: 8 x 60,000 atoms
+// 311 -> 216 us, 22 x 23,558 244 -> 238.
 template <bool CUT, bool TRIC>
 __device__ __forceinline__ int row_atoms(const Args& a, const RepDev& R, int I, int kind, float4 ci, float4 hi,
                                          const int2* ee, int e0, int e1, int lane, int* out, int cap,
